@@ -56,15 +56,11 @@ enum { B200MOE_LAYOUT_ROWS = 0, B200MOE_LAYOUT_NKI_X4 = 1 };
 enum { B200MOE_W_E4M3 = 0, B200MOE_W_E5M2 = 1, B200MOE_W_E2M1 = 5 };
 /* Variant word (`impl`) of the grouped contractions, per call.  No counterpart in the reference.
  *   B200MOE_IMPL_SIMT        CUDA-core validation kernels instead of the tensor-core path
- *   B200MOE_GEMM_TILE_N128   128 weight rows per tile instead of 256
- *   B200MOE_GEMM_NO_PAIR     never run on CTA pairs (tcgen05 cta_group::2, 256 positions x 256 weight rows)
- *   B200MOE_GEMM_FORCE_PAIR  pair an expert's 128-position tiles across its blocks whatever the block size
- *                            (default: when the block size is a multiple of 256, or experts hold four or more
- *                            tiles on average; an odd tile then ends in a half-empty pair)
- *   B200MOE_GEMM_NO_SPLIT    keep the tile an expert with an odd number of occupied tiles has left over in a
- *                            half-empty pair (default: a second, single-CTA launch takes the left-over tiles)
- *   B200MOE_GEMM_NO_OVERLAP  run that second launch strictly after the first (default: a programmatic
- *                            dependent launch that fills SMs as the first drains and finishes after it) */
+ *   B200MOE_GEMM_TILE_N128   single CTAs (128 weight rows x up to 128 tokens per tile; MX contractions only)
+ *   B200MOE_GEMM_NO_PAIR     never run on CTA pairs (tcgen05 cta_group::2, 256 weight rows x up to 256 tokens)
+ *   B200MOE_GEMM_FORCE_PAIR  CTA pairs whatever the shape (default: when the block size is a multiple of 256, or
+ *                            the block list holds two or more 128-position tiles per expert)
+ *   B200MOE_GEMM_NO_SPLIT, B200MOE_GEMM_NO_OVERLAP  accepted and ignored: there is one launch per contraction */
 enum {
   B200MOE_IMPL_SIMT = 1,
   B200MOE_GEMM_TILE_N128 = 0x100,

@@ -1,29 +1,33 @@
 // Grouped MXFP8 expert contractions on the sm_100a tensor cores.
 //
-// One persistent, warp-specialised kernel template serves both projections:
-//   warp 0      TMA producer: per 128-byte K slab, a [128 x 128B] tile of the
-//               activation rows, a [BLOCK_N x 128B] tile of the expert's weight
-//               rows (both 128B-swizzled) and their UE8M0 scale atoms (bulk copies)
-//   warp 1      allocates TMEM and issues four tcgen05.mma.kind::mxf8f6f4.block_scale
-//               (K = 32 each) per slab
-//   warps 4..7  move each slab's UE8M0 scale atoms shared memory -> registers -> TMEM
-//               (tcgen05.st, one TMEM lane quadrant per warp, one TMEM slot per pipeline
-//               stage) so the tensor pipe never spends time on tcgen05.cp
-//   warps 8..15 epilogue: two warps per TMEM lane quadrant, each thread pulls half of
-//               its accumulator row into registers with tcgen05.ld, hands the TMEM
-//               buffer back to the MMA warp at once, then works from registers
-//               EPI 0: + bias, clamp, act(gate) * up in fp32, MXFP8 re-quantisation
-//                      of the fp32 product (32 consecutive intermediates live in
-//                      one thread), codes + scale atoms out
-//               EPI 1: + bias, x routing affinity, bf16 rows out
-// Tiles are (128 positions) x (BLOCK_N weight rows); a tile's expert comes from
-// block_to_expert, padded / inactive tiles are skipped.  Tiles are enumerated
-// expert by expert, weight tile by weight tile, position tile fastest, so the
-// CTAs that run side by side read the same weight tile from L2 (a per-CTA
-// prologue derives each expert's position-tile range from block_to_expert).
-// Blocks run up to the first zero in `conditions`.  Every mbarrier wait is
-// bounded: on expiry the kernel records a code in `status`, stops issuing work
-// and tears down.
+// The weights are the M operand and the tokens the N operand of every MMA: a tile is 128 weight rows (256 on a CTA
+// pair, tcgen05 cta_group::2) times N tokens of one expert, N any multiple of 16 (32 on a pair) up to 128 (256).  An
+// expert's tokens are therefore cut into tiles of nearly equal width without padding them to 128, and one launch
+// covers every expert whatever its load.  With tokens as M (the earlier form of this kernel) an expert's last tile
+// cost a full 128 or 256 rows, odd tiles needed a second launch that streamed the weights again, and the output rows
+// left as 32-byte pieces.  Measured, whole layers, before -> now: 4096 tokens, 8 experts of 4096 x 14336, top-2: 1.36 ->
+// 1.23 ms; 8192 tokens, 256 experts of 7168 x 2048, top-8, skewed: 4.26 -> 3.91 ms; 2531 tokens, 64 experts of
+// 3072 x 1536, top-4 (160 tokens per expert): 0.53 -> 0.34 ms; 64 tokens on the first layer: 0.299 -> 0.291 ms.
+//
+// What bounds it: with many tokens the L2 -> SM feed (a pair's tile of 256 x 256 needs 64 bytes per SM and tensor-pipe
+// clock; about 48 arrive) and the power cap; with few tokens the stream of weights from HBM.
+//
+// Warp roles of a persistent CTA (512 threads):
+//   warps 0, 3, 2  TMA producers: per 128-byte K slab the weight rows (0), the token rows (3; both 128B-swizzled) and
+//               their UE8M0 scale atoms (2)
+//   warp 1      allocates TMEM, issues four tcgen05.mma.kind::mxf8f6f4.block_scale (K = 32 each) per slab
+//   warps 4..7  move each slab's scale atoms shared memory -> registers -> TMEM (tcgen05.st, one TMEM lane quadrant
+//               per warp, one TMEM slot per pipeline stage); the same bytes through tcgen05.cp cost the tensor pipe
+//               about 20 % of its cycles
+//   warps 8..15 epilogue: two groups of four warps take alternate chunks of 32 tokens.  Each thread owns one weight
+//               row (TMEM lane), pulls its part of the accumulator into registers, hands the TMEM buffer back, then
+//               EPI 0: + bias, clamp per row; the chunk is turned around in shared memory so that a thread holds 16
+//                      intermediates of one token: act(gate) * up in fp32, MXFP8 re-quantisation, codes + scales out
+//               EPI 1: (+ bias) x routing affinity to bf16, turned around in shared memory likewise so that every
+//                      token's 128 outputs leave as one 256-byte copy
+// Tiles are walked expert by expert, weight tile by weight tile, token tile fastest: CTAs that run side by side share
+// a weight tile in L2.  Blocks run up to the first zero in `conditions`.  Every mbarrier wait is bounded: on expiry
+// the kernel records a code in `status`, stops issuing work and tears down.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -32,24 +36,24 @@
 namespace b200moe {
 namespace {
 
-constexpr int kBlockM = 128;
-constexpr int kBlockK = 128;  // bytes (= e4m3 elements) per pipeline slab
+constexpr int kBlockK = 128;  // bytes per pipeline slab (128 8-bit elements, 64 bf16)
 constexpr int kGroupM = 16;
 constexpr int kMaxExperts = 512;
-constexpr int kThreads = 512;  // warp 0 producer, 1 MMA, 4-7 scale-factor movers, 8-15 epilogue (2, 3 idle)
+constexpr int kThreads = 512;
 
 struct GemmParams {
-  const uint8_t* a_sf;
-  const uint8_t* b_sf;
-  int64_t b_sf_expert_stride;
-  int b_row_atoms;  // scale atoms along the weight-row axis per expert
+  const uint8_t* x_sf;
+  const uint8_t* w_sf;
+  int64_t w_sf_expert_stride;
+  int w_row_atoms;  // scale atoms along the weight-row axis per expert
   const int32_t* block_to_expert;
   const int32_t* conditions;
-  const int32_t* tile_flags;  // per 128-position tile: non-zero if it holds a real token (NULL = all)
+  const int32_t* tile_flags;  // per 128-position tile: leading rows that can hold a token (NULL = all)
   const int32_t* tpi;
   int hidden_rows, n_blocks, B, E;
-  int m_tiles_total, n_tiles, k_blocks;
+  int m_tiles_total, k_blocks;
   int n_total;  // weight rows per expert
+  int max_n;    // tokens per tile at most
   const float* bias;
   int act;
   float gate_lo, gate_hi, up_lo, up_hi;
@@ -70,280 +74,379 @@ struct GemmParams {
   unsigned long long* clock_probe;  // optional: CTA 0 writes {SM cycles, nanoseconds} spent in the kernel
   const float* col_scale;  // dense (bf16) variant: per-expert, per-weight-row dequantisation factors [E, n_total]
                            // of fp8-row weights (NULL = none), applied to the accumulator before the bias
-  int w_format;     // element format of the weight operand (B200MOE_W_*); activations are e4m3
-  uint32_t b_tx;    // bytes one weight-tile copy reports to its mbarrier
-  int early_successor;  // 1: let the next launch in the stream begin as soon as SMs free up (it touches other rows)
-  int tile_filter;  // which position tiles a launch walks when experts are contiguous: 0 all, 1 (CTA-pair
-                    // kernel) only pairs of two live tiles, 2 (single-CTA kernel) only the tile an expert with
-                    // an odd number of live tiles has left over
-  int wait_predecessor;  // 1: launched with programmatic stream serialisation behind a launch that signalled
-                         // early; wait for that launch to finish before this grid may finish
+  int w_format;            // element format of the weight operand (B200MOE_W_*); activations are e4m3
+  int w_slab_bytes;        // bytes of a weight row per slab that a copy reports (64 for 4-bit weights)
 };
 
 // Per-CTA tile schedule, built once in shared memory.
 struct Sched {
-  int tile_start[kMaxExperts + 1];  // tiles before expert e (expert-aligned order)
-  int mt_first[kMaxExperts];        // first 128-position tile of expert e
-  int mt_count[kMaxExperts];        // its number of position tiles among the active blocks
-  int runs[kMaxExperts];            // how many separate block runs expert e has (1 when sorted); after the
-                                    // build, in left-over mode: the expert of left-over tile i
-  int n_live[kMaxExperts];          // 1 + index (among the expert's tiles) of its last tile that holds a token
-  int left_m[kMaxExperts];          // left-over mode: position tile of left-over i
-  int n_left;                       // left-over mode: number of left-over tiles
-  int n_full;                       // tiles [0, n_full) are whole; each later index is half (128 weight rows) of
-                                    // one of the tiles that would not fill a last round of CTAs
-  int n_active;                     // blocks before the first zero condition
-  int contiguous;                   // every expert's blocks are adjacent
-  int total;                        // number of tiles to walk
+  int start[kMaxExperts + 1];  // token tiles before expert e
+  int first_row[kMaxExperts];  // first position of expert e
+  int rows[kMaxExperts];       // positions from there to its last token; negative: an inner 128-row tile is not full,
+                               // and the expert is walked in windows of 128 positions instead
+  int n_active;                // blocks before the first zero condition
+  int contiguous;              // every expert's blocks are adjacent
+  int h, w_tiles;              // weight rows per tile, tiles per expert
+  int n_full, parts;           // tiles [0, n_full) are whole; each later index is one of `parts` equal row ranges of a
+                               // tile that would not fill a last round of CTAs
+  int total;                   // number of tiles to walk
+  int stages, x_bytes;         // single CTA: pipeline depth and bytes of token rows per slab
 };
 
-// `mg` = position tiles per scheduling unit (1, or 2 when a CTA pair shares a weight tile).
-// `halves`: single-CTA launches with 256-row weight tiles may cut the tiles of a partly filled last round in two.
-__device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int mg, bool halves, int n_units) {
+__device__ __forceinline__ int round_up(int v, int m) { return (v + m - 1) / m * m; }
+
+__device__ __forceinline__ int token_tiles(const GemmParams& p, int rows) {
+  return rows < 0 ? (-rows + 127) >> 7 : (rows + p.max_n - 1) / p.max_n;
+}
+
+// CTAS 2: 256 weight rows per tile.  CTAS 1: 128, or fewer where that spreads the rows more evenly over the CTAs
+// (a decode launch is bound by streaming weights, so its time is the largest number of rows any CTA gets): e.g. 8
+// experts x 4096 rows on 148 CTAs are 1.73 rounds of 128-row tiles, but exactly two rounds of 112-row tiles.
+//
+// Everything read from global memory here is fetched at once into `scratch` (shared memory the pipeline will use
+// later, `scratch_ints` long; larger problems read global memory again): the prologue costs one memory latency, which
+// is what a decode launch of a few tens of microseconds notices.
+template <int CTAS, int EPI>
+__device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n_units, int* scratch, int scratch_ints,
+                                            int ring_bytes, int slab_fixed_bytes, int max_stages) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int sub = p.B >> 7;
   if (tid == 0) { s.n_active = p.n_blocks; s.contiguous = 1; }
-  for (int e = tid; e < p.E; e += nthr) { s.mt_first[e] = 0; s.mt_count[e] = 0; s.runs[e] = 0; }
+  for (int e = tid; e < p.E; e += nthr) { s.first_row[e] = 0; s.rows[e] = 0; s.start[e] = 0; }
   __syncthreads();
-  if (p.conditions != nullptr)
-    for (int b = tid; b < p.n_blocks; b += nthr)
-      if (p.conditions[b] == 0) atomicMin(&s.n_active, b);
+  const int32_t* b2e = p.block_to_expert;
+  const int32_t* flags = p.tile_flags;
+  const bool staged = p.n_blocks + p.m_tiles_total <= scratch_ints;
+  for (int b = tid; b < p.n_blocks; b += nthr) {
+    const int e = staged ? p.block_to_expert[b] : 0;
+    const int run = p.conditions != nullptr ? p.conditions[b] : 1;
+    if (staged) scratch[b] = e;
+    if (run == 0) atomicMin(&s.n_active, b);
+  }
+  if (staged) {
+    if (p.tile_flags != nullptr) {
+      for (int t = tid; t < p.m_tiles_total; t += nthr) scratch[p.n_blocks + t] = p.tile_flags[t];
+      flags = scratch + p.n_blocks;
+    }
+    b2e = scratch;
+  }
   __syncthreads();
   const int n_active = s.n_active;
+  // start[] counts an expert's separate runs of blocks here, rows[] its 128-row tiles
   for (int b = tid; b < n_active; b += nthr) {
-    const int e = p.block_to_expert[b];
+    const int e = b2e[b];
     if (e < 0 || e >= p.E) continue;
-    if (b == 0 || p.block_to_expert[b - 1] != e) {
-      s.mt_first[e] = b * sub;
-      if (atomicAdd(&s.runs[e], 1) > 0) s.contiguous = 0;
+    if (b == 0 || b2e[b - 1] != e) {
+      s.first_row[e] = b * p.B;
+      if (atomicAdd(&s.start[e], 1) > 0) s.contiguous = 0;
     }
-    atomicAdd(&s.mt_count[e], sub);
+    atomicAdd(&s.rows[e], sub);
   }
   __syncthreads();
-  for (int e = tid; e < p.E; e += nthr) {
-    int live = s.mt_count[e];
-    if (p.tile_flags != nullptr)
-      while (live > 0 && p.tile_flags[s.mt_first[e] + live - 1] == 0) --live;
-    s.n_live[e] = live;
+  const bool contiguous = s.contiguous;
+  for (int e = tid; e < p.E && contiguous; e += nthr) {
+    int live = s.rows[e], last = 128;
+    if (flags != nullptr && live > 0) {
+      const int t0 = s.first_row[e] >> 7;
+      while (live > 0 && (last = flags[t0 + live - 1]) == 0) --live;
+    }
+    s.rows[e] = live > 0 ? (live - 1) * 128 + last : 0;
   }
   __syncthreads();
-  if (tid == 0) {
-    int run = 0, n_left = 0;
-    const bool leftovers = s.contiguous && p.tile_filter == 2;
-    for (int e = 0; e < p.E; ++e) {
-      s.tile_start[e] = run;
-      if (s.contiguous && p.tile_filter == 1) {
-        run += (s.n_live[e] / 2) * p.n_tiles;                // full pairs only; the odd tile goes to the other launch
-      } else if (leftovers) {
-        if (s.n_live[e] & 1) { s.left_m[n_left] = s.mt_first[e] + s.n_live[e] - 1; s.runs[n_left] = e; ++n_left; }
-      } else {
-        run += ((s.mt_count[e] + mg - 1) / mg) * p.n_tiles;  // an odd tile count leaves the last pair half empty
+  if (flags != nullptr && contiguous) {
+    for (int t = tid; t < n_active * sub; t += nthr) {
+      if (flags[t] >= 128) continue;
+      const int e = b2e[t / sub];
+      if (e < 0 || e >= p.E) continue;
+      const int r = s.rows[e], end = s.first_row[e] + (r < 0 ? -r : r);
+      if ((t + 1) * 128 < end && r > 0) atomicMin(&s.rows[e], -r);
+    }
+    __syncthreads();
+  }
+  if (tid < 32) {
+    int run = 0, widest = 0;
+    for (int e0 = 0; e0 < p.E; e0 += 32) {
+      const int e = e0 + tid;
+      const int rows = e < p.E ? s.rows[e] : 0;
+      const int own = token_tiles(p, rows);
+      if (rows != 0) widest = max(widest, rows < 0 ? 128 : (rows + own - 1) / own);
+      int v = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (tid >= o) v += u;
       }
+      if (e < p.E) s.start[e] = run + v - own;
+      run += __shfl_sync(0xffffffffu, v, 31);
     }
-    s.n_left = n_left;
-    if (leftovers) run = n_left * p.n_tiles;
-    if (!s.contiguous && p.tile_filter == 2) run = 0;        // scattered blocks: the pair launch does everything
-    s.tile_start[p.E] = run;
-    // scattered blocks: pairs stay inside a block when it holds an even number of tiles, else every tile is
-    // a unit of its own (the pair's second CTA idles)
-    const int units = (mg == 2 && (sub & 1)) ? p.m_tiles_total : p.m_tiles_total / mg;
-    s.total = (s.contiguous || p.tile_filter == 2) ? run : units * p.n_tiles;
-    s.n_full = s.total;
-    if (halves && (s.contiguous || p.tile_filter == 2) && s.total >= 2 * n_units) {
-      // whole rounds of n_units tiles keep their width; if the rest fits one round even when cut in two, cut it:
-      // the last round then takes half as long
-      const int whole = (s.total / n_units) * n_units, rest = s.total - whole;
-      if (rest > 0 && 2 * rest <= n_units) { s.n_full = whole; s.total = whole + 2 * rest; }
+    widest = contiguous ? static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<uint32_t>(widest))) : 128;
+    const int tok_tiles = contiguous ? run : n_active * sub;
+    int h = 128 * CTAS, parts = 1, stages = max_stages, x_bytes = 0;
+    if constexpr (CTAS == 1) {
+      // one candidate height per lane: 128, 128 - kGran, ... (MX blocks of 32 intermediates need whole groups of 32
+      // gate and 32 up rows).  Heights under 96 keep too few bytes in flight and are only taken when they leave
+      // far fewer rows on the fullest CTA.
+      constexpr int kGran = EPI == 0 ? 64 : 16;
+      const int c = 128 - tid * kGran;
+      uint32_t key = 0xffffffffu;
+      if (c >= (EPI == 0 ? 64 : 32)) {
+        const int tiles = tok_tiles * ((p.n_total + c - 1) / c);
+        const int whole = tiles / n_units, rest = tiles - whole * n_units;
+        int cut = 1;
+        if (rest > 0)
+          for (int q = 2; q * kGran <= c && rest * q <= n_units; ++q)
+            if (c % (q * kGran) == 0) cut = q;
+        const int cost = whole * max(c, 88) + (rest > 0 ? c / cut : 0);
+        key = (static_cast<uint32_t>(min(cost, 0x3fffff)) << 10) | static_cast<uint32_t>(tid << 5) | static_cast<uint32_t>(cut);
+      }
+      key = __reduce_min_sync(0xffffffffu, key);
+      h = 128 - static_cast<int>((key >> 5) & 31) * kGran;
+      parts = static_cast<int>(key & 31);
+      // narrow token tiles leave room for a deeper ring of weight slabs
+      x_bytes = max(round_up(widest, 16), 16) * kBlockK;
+      stages = min(max_stages, ring_bytes / (x_bytes + slab_fixed_bytes));
+    }
+    if (tid == 0) {
+      s.start[p.E] = run;
+      s.h = h;
+      s.w_tiles = (p.n_total + h - 1) / h;
+      s.parts = parts;
+      s.stages = stages;
+      s.x_bytes = x_bytes;
+      const int tiles = tok_tiles * s.w_tiles;
+      s.n_full = parts > 1 ? tiles / n_units * n_units : tiles;
+      s.total = s.n_full + (tiles - s.n_full) * parts;
     }
   }
   __syncthreads();
 }
 
-// m_tile is the first position tile of the unit; with mg == 2 the pair's CTAs take m_tile and m_tile + 1, and
-// `second` says whether m_tile + 1 is a tile of the same expert that holds tokens (an expert with an odd number
-// of tiles ends in a half-empty pair: its second CTA still supplies half of the weight tile but copies no
-// activations and writes nothing).
-// `part`: -1 for a whole weight tile, 0 / 1 for its first / second 128 rows (see Sched::n_full).
-__device__ __forceinline__ bool decode_tile(const GemmParams& p, const Sched& s, int tile, int mg, int& m_tile,
-                                            int& n_tile, int& expert, int& second, int& part) {
-  second = mg == 2 ? 1 : 0;
-  part = -1;
+// A tile: token rows [row0, row0 + n) of the position axis, weight rows [w_row0, w_row0 + w_rows) of `expert`.
+struct TileRec {
+  int row0, w_row0, expert;
+  int shape;  // bits 0-9 n, bits 10-19 w_rows; 0 = nothing to do
+  __device__ __forceinline__ int n() const { return shape & 1023; }
+  __device__ __forceinline__ int w_rows() const { return shape >> 10; }
+};
+
+template <int CTAS>
+__device__ __forceinline__ TileRec decode_tile(const GemmParams& p, const Sched& s, int tile) {
+  constexpr int kStepN = CTAS == 2 ? 32 : 16;
+  int sub_part = 0;
+  bool cut = false;
   if (tile >= s.n_full) {
-    part = (tile - s.n_full) & 1;
-    tile = s.n_full + ((tile - s.n_full) >> 1);
+    cut = true;
+    sub_part = (tile - s.n_full) % s.parts;
+    tile = s.n_full + (tile - s.n_full) / s.parts;
   }
-  if (s.contiguous && p.tile_filter == 2) {
-    const int i = tile % s.n_left;
-    m_tile = s.left_m[i];
-    expert = s.runs[i];
-    n_tile = tile / s.n_left;
-    return true;
-  }
+  int e, w_tile, row0, n;
   if (s.contiguous) {
     int lo = 0, hi = p.E;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (s.tile_start[mid] <= tile) lo = mid; else hi = mid;
+      if (s.start[mid] * s.w_tiles <= tile) lo = mid; else hi = mid;
     }
-    expert = lo;
-    const int local = tile - s.tile_start[lo];
-    const int cnt = p.tile_filter == 1 ? s.n_live[lo] / 2 : (s.mt_count[lo] + mg - 1) / mg;
-    const int idx = local % cnt;
-    m_tile = s.mt_first[lo] + idx * mg;
-    n_tile = local / cnt;
-    if (mg == 2 && idx * 2 + 1 >= s.mt_count[lo]) second = 0;
+    e = lo;
+    const int local = tile - s.start[e] * s.w_tiles;
+    const int cnt = s.start[e + 1] - s.start[e];
+    const int t = local % cnt;
+    w_tile = local / cnt;
+    const int rows = s.rows[e];
+    if (rows < 0) {
+      row0 = s.first_row[e] + t * 128;
+      n = p.tile_flags[row0 >> 7];
+      if (n > p.max_n) n = p.max_n;  // (max_n is at least 128)
+    } else {
+      const int width = round_up((rows + cnt - 1) / cnt, kStepN);
+      row0 = s.first_row[e] + t * width;
+      n = min(width, rows - t * width);
+    }
   } else {
-    const bool solo = mg == 2 && ((p.B >> 7) & 1);
-    if (solo) { mg = 1; second = 0; }
-    const int units = p.m_tiles_total / mg;
-    const int per_group = kGroupM * p.n_tiles;
+    // scattered blocks: one tile per 128 positions, in the given order
+    const int units = s.n_active * (p.B >> 7);
+    const int per_group = kGroupM * s.w_tiles;
     const int g = tile / per_group;
-    const int first_m = g * kGroupM;
-    const int gs = min(kGroupM, units - first_m);
+    const int first = g * kGroupM;
+    const int gs = min(kGroupM, units - first);
     const int within = tile - g * per_group;
-    m_tile = (first_m + within % gs) * mg;
-    n_tile = within / gs;
-    const int block = m_tile / (p.B >> 7);
-    if (block >= s.n_active) return false;
-    expert = p.block_to_expert[block];
-    if (expert < 0 || expert >= p.E) return false;
+    const int m_tile = first + within % gs;
+    w_tile = within / gs;
+    e = p.block_to_expert[m_tile / (p.B >> 7)];
+    row0 = m_tile * 128;
+    n = (e < 0 || e >= p.E) ? 0 : (p.tile_flags ? p.tile_flags[m_tile] : 128);
   }
-  if (p.tile_flags != nullptr) {
-    if (second && p.tile_flags[m_tile + 1] == 0) second = 0;
-    if (p.tile_flags[m_tile] == 0 && !second) return false;
-  }
-  return true;
+  const int h = cut ? s.h / s.parts : s.h;
+  const int w_row0 = w_tile * s.h + sub_part * h;
+  const int w_rows = min(h, p.n_total - w_row0);
+  if (n <= 0 || w_rows <= 0) return TileRec{0, 0, 0, 0};
+  return TileRec{row0, w_row0, e, round_up(n, kStepN) | (w_rows << 10)};
 }
 
-// Activation rows worth copying for a 128-position tile: tile_flags holds the number of leading rows that can
-// carry a token (tokens fill a block from its start), so short tiles -- decode, the last block of an expert --
-// copy a 32- or 64-row box.  The MMA still spans 128 rows; what it computes from the stale rows below the box
-// lands in rows nobody reads.
-__device__ __forceinline__ int tile_copy_rows(const GemmParams& p, int m_tile) {
-  if (p.tile_flags == nullptr) return kBlockM;
-  const int f = p.tile_flags[m_tile];
-  return f <= 0 ? 0 : (f <= 32 ? 32 : (f <= 64 ? 64 : kBlockM));
-}
+// A CTA's own tiles, decoded once in the prologue by all threads (the decode -- a search over the experts, divisions,
+// tile_flags reads -- costs about a thousand clocks, which the MMA-issuing thread would otherwise spend at every tile
+// boundary with the tensor pipe idle); tiles past the table are decoded on the spot.
+constexpr int kTileTable = 256;
 
-// A CTA's own tiles, decoded once in the prologue by all threads: the per-tile decode (a search over the experts,
-// two divisions, tile_flags reads from global memory) costs about a thousand clocks, which the single MMA-issuing
-// thread would otherwise spend at every tile boundary with the tensor pipe idle.
-struct TileRec {
-  int m_tile, n_tile, expert;
-  int flags;  // bit 0 valid, bit 1 second, bits 2-3 part + 1, bits 8-15 / 16-23 activation rows to copy (lead / peer)
-};
-constexpr int kTileTable = 448;  // entries per CTA (7 KB); later tiles are decoded on the spot
-
-__device__ __forceinline__ bool fetch_tile(const GemmParams& p, const Sched& s, const TileRec* table, int it, int tile,
-                                           int mg, int& m_tile, int& n_tile, int& expert, int& second, int& part,
-                                           int& rows_lead, int& rows_peer) {
+template <int CTAS>
+__device__ __forceinline__ TileRec fetch_tile(const GemmParams& p, const Sched& s, const TileRec* table, int it, int tile) {
   if (it < kTileTable) {
     const int4 r = *reinterpret_cast<const int4*>(table + it);
-    if (!(r.w & 1)) return false;
-    m_tile = r.x;
-    n_tile = r.y;
-    expert = r.z;
-    second = (r.w >> 1) & 1;
-    part = ((r.w >> 2) & 3) - 1;
-    rows_lead = (r.w >> 8) & 0xff;
-    rows_peer = (r.w >> 16) & 0xff;
-    return true;
+    return TileRec{r.x, r.y, r.z, r.w};
   }
-  if (!decode_tile(p, s, tile, mg, m_tile, n_tile, expert, second, part)) return false;
-  rows_lead = tile_copy_rows(p, m_tile);
-  rows_peer = second ? tile_copy_rows(p, m_tile + 1) : 0;
-  return true;
+  return decode_tile<CTAS>(p, s, tile);
 }
 
-template <int BLOCK_N, int STAGES, int CTAS = 1>
+// Chunk buffer of the gate/up epilogue: 32 tokens x 128 weight rows of fp32, token-major.  Rows 64.. sit 8 words
+// further on and a token's row is 140 words, so that the 16-byte reads of eight neighbouring threads (two tokens x
+// four row ranges) touch 32 different banks, as do the 4-byte writes of 32 neighbouring rows.
+constexpr int kTurnPitch = 140;
+constexpr int kTurnBytes = 32 * kTurnPitch * 4;
+// The down epilogue's: 32 tokens x 128 output columns of bf16, a token's row 272 bytes so that the eight 16-byte rows of
+// a transposing matrix store touch 32 different banks; two buffers, so that one is filled while the other is copied out.
+constexpr int kRowPitch = 272;
+constexpr int kRowBytes = 32 * kRowPitch;
+
+template <int EPI, int CTAS>
 struct SmemLayout {
-  static constexpr int kA = kBlockM * kBlockK;
-  static constexpr int kB = (BLOCK_N / CTAS) * kBlockK;  // a CTA pair splits the weight rows
-  static constexpr int kSfa = 512;
-  static constexpr int kSfbAtoms = BLOCK_N > 128 ? 2 : 1;
-  static constexpr int kSfb = kSfbAtoms * 512;
-  static constexpr int kOffA = 0;
-  static constexpr int kOffB = kOffA + STAGES * kA;
-  static constexpr int kOffSfa = kOffB + STAGES * kB;
-  static constexpr int kOffSfb = kOffSfa + STAGES * kSfa;
-  static constexpr int kOffBar = kOffSfb + STAGES * kSfb;
-  static constexpr int kOffSched = kOffBar + 256;
+  static constexpr int kMaxN = CTAS == 2 ? 256 : 128;
+  static constexpr int kMaxStages = CTAS == 2 ? 5 : 8;
+  static constexpr int kW = 128 * kBlockK;
+  static constexpr int kX = (kMaxN / CTAS) * kBlockK;  // a CTA pair splits the token rows
+  static constexpr int kSfwAtoms = CTAS == 2 ? 1 : 2;  // weight rows of a single CTA may start inside an atom
+  static constexpr int kSfxAtoms = kMaxN / 128 + 1;    // so may token rows
+  static constexpr int kSf = (kSfwAtoms + kSfxAtoms) * 512;
+  static constexpr int kRing = CTAS == 2 ? kMaxStages * (kW + kX + kSf) : 180 * 1024;
+  // per epilogue group: the chunk buffer(s); EPI 1 also the affinity and the destination row of each of its tokens
+  static constexpr int kGroup = EPI == 0 ? kTurnBytes : 2 * kRowBytes + (kMaxN / 2) * 8;
+  static constexpr int kOffEpi = kRing;
+  static constexpr int kOffBar = kOffEpi + 2 * kGroup;
+  static constexpr int kOffSched = kOffBar + 384;
   static constexpr int kOffTiles = (kOffSched + static_cast<int>(sizeof(Sched)) + 15) & ~15;
   static constexpr int kBytes = kOffTiles + kTileTable * static_cast<int>(sizeof(TileRec)) + 1024;  // + alignment slack
+  static_assert(kGroup % 16 == 0 && kRing % 1024 == 0, "alignment of the epilogue buffers");
 };
+
+// Two accumulators of 224 columns (single CTA: 128), used in turn, so that a tile's MMAs run while the epilogue drains
+// the one before; a tile of more than 224 tokens takes both.  The MMA issuer and the epilogue walk the same sequence.
+struct AccCursor {
+  uint32_t taken[2] = {0, 0}, filled[2] = {0, 0};  // phase parities of tmem_empty / tmem_full
+  int next = 0;
+  __device__ __forceinline__ int begin(bool wide) { return wide ? 0 : next; }
+  __device__ __forceinline__ void end(bool wide) {
+    if (wide) {
+      taken[0] ^= 1u;
+      taken[1] ^= 1u;
+      filled[0] ^= 1u;
+      next = 0;
+    } else {
+      if (next == 0) { taken[0] ^= 1u; filled[0] ^= 1u; }
+      else { taken[1] ^= 1u; filled[1] ^= 1u; }
+      next ^= 1;
+    }
+  }
+};
+
+__device__ __forceinline__ void group_barrier(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+// All 128 threads of an epilogue group agree whether the wait succeeded.
+__device__ __forceinline__ bool group_all(int id, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %1, 0;\n"
+      "bar.red.and.pred q, %2, 128, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(ok ? 1 : 0), "r"(id)
+      : "memory");
+  return r != 0;
+}
+
+// act(gate) * up for 16 intermediates of one token; returns the largest |product| as bits.
+__device__ __forceinline__ uint32_t swiglu16(float (&g)[16], const float (&u)[16], int act) {
+  switch (act) {
+    case B200MOE_ACT_SILU:
+#pragma unroll
+      for (int j = 0; j < 16; ++j) g[j] = __fdividef(g[j], 1.0f + __expf(-g[j])) * u[j];
+      break;
+    case B200MOE_ACT_SWISH:
+#pragma unroll
+      for (int j = 0; j < 16; ++j) g[j] = apply_act(g[j], B200MOE_ACT_SWISH) * u[j];
+      break;
+    case B200MOE_ACT_GELU:
+#pragma unroll
+      for (int j = 0; j < 16; ++j) g[j] = apply_act(g[j], B200MOE_ACT_GELU) * u[j];
+      break;
+    default:
+#pragma unroll
+      for (int j = 0; j < 16; ++j) g[j] = apply_act(g[j], B200MOE_ACT_GELU_TANH) * u[j];
+      break;
+  }
+  uint32_t mx = 0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) mx = max(mx, __float_as_uint(g[j]) & 0x7fffffffu);
+  return mx;
+}
 
 // KIND 0: MXFP8 activations x MX weights, block-scaled MMAs (kind::mxf8f6f4.block_scale).
 // KIND 1: bf16 activations x bf16 weights (kind::f16), the reference's non-MX variants: no scale atoms travel, the
 //         four scale-mover warps idle, the gate/up epilogue writes bf16 intermediates instead of MX codes.  Operand
 //         rows are addressed in bytes, so a 128-byte slab is 64 bf16 elements = four K = 16 MMAs.
-template <int BLOCK_N, int STAGES, int EPI, int CTAS, int KIND = 0>
+// CTAS 2: the two CTAs of a cluster form one tcgen05 cta_group::2 unit.  Each loads its own 128 weight rows and half of
+//         the token rows; the even CTA issues M = 256 MMAs that read both CTAs' shared memory and write both CTAs'
+//         TMEM, so a token row crosses L2 -> SM once per 256 weight rows.
+struct WeightMaps { CUtensorMap rows128, rows64, rows32, rows16; };
+struct TokenMaps { CUtensorMap rows128, rows64, rows32, rows16; };
+
+template <int EPI, int CTAS, int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
-grouped_mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a64,
-                          const __grid_constant__ CUtensorMap tmap_a32, const __grid_constant__ CUtensorMap tmap_b,
-                          const __grid_constant__ CUtensorMap tmap_b128, const __grid_constant__ CUtensorMap tmap_sfa,
-                          const __grid_constant__ CUtensorMap tmap_sfb, const GemmParams p) {
-  // CTAS == 2: the two CTAs of a cluster form one tcgen05 cta_group::2 unit.  Each loads its own 128
-  // activation rows and half of the weight tile; the even CTA issues M = 256 MMAs that read both CTAs'
-  // shared memory and write both CTAs' TMEM, so a weight byte crosses L2 -> SM once per 256 rows.
-  using L = SmemLayout<BLOCK_N, STAGES, CTAS>;
-  constexpr int kAcc = (BLOCK_N <= 128) ? 2 : 1;
-  constexpr int kSfCol = kAcc * BLOCK_N;  // TMEM columns: accumulators, then SFA (4), then SFB
+grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_constant__ TokenMaps xmap,
+                          const __grid_constant__ CUtensorMap sfw_map, const __grid_constant__ CUtensorMap sfx_map,
+                          const GemmParams p) {
+  using L = SmemLayout<EPI, CTAS>;
+  constexpr int kMaxStages = L::kMaxStages;
+  constexpr int kChunks = L::kMaxN / 64;   // 32-token chunks per epilogue group
+  constexpr int kAccStride = CTAS == 2 ? 224 : 128;
+  constexpr int kSfCol = 448;              // TMEM columns: accumulators, then per stage 4 of weight and 4 / 8 of token scales
+  constexpr int kSfSlot = CTAS == 2 ? 12 : 8;
+  static_assert(kSfCol + kMaxStages * kSfSlot <= 512, "scale slots exceed TMEM");
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kIdesc = KIND == 0 ? make_idesc(kBlockM * CTAS, BLOCK_N) : make_idesc_bf16(kBlockM * CTAS, BLOCK_N);
-  // operand bytes per stage (scale atoms report to sf_full) depend on the tile: short activation boxes, and
-  // 4-bit weights that land in the same padded 128-byte rows but report their packed size
-  const uint32_t idesc_base = KIND == 0 ? (kIdesc | (static_cast<uint32_t>(p.w_format) << 10)) : kIdesc;
+  // M is fixed; N is or-ed in per tile
+  const uint32_t idesc_base = KIND == 0 ? (make_idesc(128 * CTAS, 0) | (static_cast<uint32_t>(p.w_format) << 7))
+                                        : make_idesc_bf16(128 * CTAS, 0);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* full = bars;
-  uint64_t* empty = bars + STAGES;
-  uint64_t* tmem_full = bars + 2 * STAGES;
-  uint64_t* tmem_empty = bars + 2 * STAGES + kAcc;
-  uint64_t* sf_full = bars + 2 * STAGES + 2 * kAcc;             // scale atoms of a stage landed (per CTA)
-  uint64_t* sf_ready = bars + 3 * STAGES + 2 * kAcc;            // ... and sit in their TMEM slot (pair leader)
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 4 * STAGES + 2 * kAcc);
+  uint64_t* empty = bars + kMaxStages;
+  uint64_t* sf_full = bars + 2 * kMaxStages;   // scale atoms of a stage landed (per CTA)
+  uint64_t* sf_ready = bars + 3 * kMaxStages;  // ... and sit in their TMEM slot (pair leader)
+  uint64_t* tmem_full = bars + 4 * kMaxStages;
+  uint64_t* tmem_empty = bars + 4 * kMaxStages + 2;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 4 * kMaxStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
   Sched& sched = *reinterpret_cast<Sched*>(smem + L::kOffSched);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform to the compiler
+  const int lane = threadIdx.x & 31;
   long long probe_c0 = 0;
   unsigned long long probe_t0 = 0;
   if (p.clock_probe != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
     probe_c0 = clock64();
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(probe_t0));
   }
-  // The left-over launch that follows a CTA-pair launch works on different rows of the same buffers: it may start
-  // on every SM this launch no longer needs (programmatic dependent launch).  The successor does its tiles without
-  // waiting and executes griddepcontrol.wait before it exits, so it never completes before this grid has.
-  if (p.early_successor && threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int cta_rank = CTAS == 2 ? static_cast<int>(cluster_cta_rank()) : 0;
   const int unit = blockIdx.x / CTAS, n_units = gridDim.x / CTAS;
-  build_sched(p, sched, CTAS, CTAS == 1 && BLOCK_N == 256, n_units);
-  const int total_tiles = sched.total;
-  TileRec* tile_table = reinterpret_cast<TileRec*>(smem + L::kOffTiles);
-  for (int i = threadIdx.x; i < kTileTable; i += kThreads) {
-    const int tile = unit + i * n_units;
-    TileRec r{0, 0, 0, 0};
-    if (tile < total_tiles) {
-      int m_tile, n_tile, e, second, part;
-      if (decode_tile(p, sched, tile, CTAS, m_tile, n_tile, e, second, part)) {
-        const int rl = tile_copy_rows(p, m_tile), rp = second ? tile_copy_rows(p, m_tile + 1) : 0;
-        r = TileRec{m_tile, n_tile, e, 1 | (second << 1) | ((part + 1) << 2) | (rl << 8) | (rp << 16)};
-      }
-    }
-    tile_table[i] = r;  // read after the __syncthreads below
-  }
-
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
       mbar_init(&sf_full[s], 1);
       mbar_init(&sf_ready[s], 4 * CTAS);
     }
-    for (int a = 0; a < kAcc; ++a) {
+    for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
       mbar_init(&tmem_empty[a], 8 * CTAS);
     }
@@ -364,182 +467,283 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
   }
+  build_sched<CTAS, EPI>(p, sched, n_units, reinterpret_cast<int*>(smem), L::kRing / 4, L::kRing, L::kW + L::kSf, kMaxStages);
+  const int total_tiles = sched.total;
+  const int stages = CTAS == 2 ? kMaxStages : sched.stages;
+  const int x_stage = CTAS == 2 ? L::kX : sched.x_bytes;
+  const int off_x = stages * L::kW, off_sf = off_x + stages * x_stage;
+  TileRec* tile_table = reinterpret_cast<TileRec*>(smem + L::kOffTiles);
+  for (int i = threadIdx.x; i < kTileTable; i += kThreads) {
+    const int tile = unit + i * n_units;
+    if (tile < total_tiles) tile_table[i] = decode_tile<CTAS>(p, sched, tile);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the prologue's scratch becomes the copies' target
   tc_fence_before();
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync_all();  // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  // Register budget per warpgroup (4 warps): the epilogue warps hold 128 accumulator values per thread,
+  // Register budget per warpgroup (4 warps): the epilogue warps hold up to 128 accumulator values per thread,
   // everyone else needs few.  512 threads x 128 at launch = 2 x 128 x 64 + 2 x 128 x 192.
   if (warp < 4) {
     reg_dec<64>();
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    // Each of these warps walks its loop as a whole, with warp-uniform values, and one elected lane issues: a lone
+    // thread pays about a hundred clocks per copy for moving the operands of one instruction into uniform registers,
+    // and three copies' worth per slab more than the slab's MMAs take, which is why the copies have three warps.
+    const bool leader = elect_one();
+    if (warp != 1) {
+      // ---------------------------------------------------------- TMA producers
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      constexpr int kRowsB = BLOCK_N / CTAS;  // weight rows this CTA copies per slab
       for (int tile = unit, it = 0; tile < total_tiles && ok; tile += n_units, ++it) {
-        int m_tile, n_tile, e, second, part, rows_lead, rows_peer;
-        if (!fetch_tile(p, sched, tile_table, it, tile, CTAS, m_tile, n_tile, e, second, part, rows_lead, rows_peer))
-          continue;
-        m_tile += cta_rank;
-        const int my_rows = cta_rank == 0 ? rows_lead : rows_peer;
-        const CUtensorMap* map_a = my_rows == 32 ? &tmap_a32 : (my_rows == 64 ? &tmap_a64 : &tmap_a);
-        // a half tile (single-CTA launches only) copies 128 weight rows through the 128-row map
-        const int n_row0 = n_tile * BLOCK_N + (part > 0 ? BLOCK_N / 2 : 0);
-        const uint32_t b_bytes = part >= 0 ? p.b_tx / 2 : p.b_tx;
-        const uint32_t stage_bytes = static_cast<uint32_t>(rows_lead + rows_peer) * kBlockK + CTAS * b_bytes;
-        const int atom0 = n_row0 >> 7;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
-          // scale atoms of this CTA's rows and of the whole weight tile -> this CTA's own barrier
-          // (rows past the end of the atom table read as zero and still count their bytes)
-          if constexpr (KIND == 0) {
-            mbar_expect_tx(&sf_full[stage], L::kSfa + L::kSfb);
-            tma_load_2d(smem + L::kOffSfa + stage * L::kSfa, &tmap_sfa, 0, m_tile * p.k_blocks + kb, &sf_full[stage]);
-#pragma unroll
-            for (int j = 0; j < L::kSfbAtoms; ++j)
-              tma_load_2d(smem + L::kOffSfb + stage * L::kSfb + j * 512, &tmap_sfb, 0,
-                          (e * p.b_row_atoms + atom0 + j) * p.k_blocks + kb, &sf_full[stage]);
+        const TileRec r = fetch_tile<CTAS>(p, sched, tile_table, it, tile);
+        if (r.shape == 0 || (KIND != 0 && warp == 2)) continue;
+        const int w_row0 = r.w_row0 + cta_rank * 128;
+        // a pair always copies 2 x 128 weight rows (rows past the end read as zero)
+        const int w_copy = CTAS == 2 ? 128 : round_up(r.w_rows(), 16);
+        if (warp == 0) {
+          // weight rows; the even CTA's barrier counts both CTAs' operand bytes of a pair
+          const uint32_t stage_bytes = static_cast<uint32_t>(CTAS * w_copy * p.w_slab_bytes + r.n() * kBlockK);
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
+            uint8_t* ws = smem + stage * L::kW;
+            if (leader) {
+              if (cta_rank == 0) mbar_expect_tx(&full[stage], stage_bytes);
+              if constexpr (CTAS == 2) {
+                tma2_load_3d(ws, &wmap.rows128, kb * kBlockK, w_row0, r.expert, &full[stage]);
+              } else if (w_copy == 128) {
+                tma_load_3d(ws, &wmap.rows128, kb * kBlockK, w_row0, r.expert, &full[stage]);
+              } else {
+                int at = 0;
+                if (w_copy & 64) { tma_load_3d(ws, &wmap.rows64, kb * kBlockK, w_row0, r.expert, &full[stage]); at = 64; }
+                if (w_copy & 32) { tma_load_3d(ws + at * kBlockK, &wmap.rows32, kb * kBlockK, w_row0 + at, r.expert, &full[stage]); at += 32; }
+                if (w_copy & 16) tma_load_3d(ws + at * kBlockK, &wmap.rows16, kb * kBlockK, w_row0 + at, r.expert, &full[stage]);
+              }
+            }
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
           }
-          if constexpr (CTAS == 2) {
-            // operand tiles of both CTAs complete on the even CTA's barrier
-            if (cta_rank == 0) mbar_expect_tx(&full[stage], stage_bytes);
-            if (my_rows > 0)
-              tma2_load_2d(smem + L::kOffA + stage * L::kA, map_a, kb * kBlockK, m_tile * kBlockM, &full[stage]);
-            tma2_load_3d(smem + L::kOffB + stage * L::kB, &tmap_b, kb * kBlockK,
-                         n_tile * BLOCK_N + cta_rank * (BLOCK_N / 2), e, &full[stage]);
-          } else {
-            mbar_expect_tx(&full[stage], stage_bytes);
-            if (my_rows > 0)
-              tma_load_2d(smem + L::kOffA + stage * L::kA, map_a, kb * kBlockK, m_tile * kBlockM, &full[stage]);
-            tma_load_3d(smem + L::kOffB + stage * L::kB, part >= 0 ? &tmap_b128 : &tmap_b, kb * kBlockK, n_row0, e,
-                        &full[stage]);
+        } else if (warp == 3) {
+          // token rows
+          const int n_cta = r.n() / CTAS, x_row0 = r.row0 + cta_rank * n_cta;
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
+            uint8_t* xs = smem + off_x + stage * x_stage;
+            if (leader) {
+              auto load_x = [&](const CUtensorMap& map, int at) {
+                if constexpr (CTAS == 2) tma2_load_2d(xs + at * kBlockK, &map, kb * kBlockK, x_row0 + at, &full[stage]);
+                else tma_load_2d(xs + at * kBlockK, &map, kb * kBlockK, x_row0 + at, &full[stage]);
+              };
+              int at = 0;
+              if (n_cta & 128) { load_x(xmap.rows128, 0); at = 128; }
+              if (n_cta & 64) { load_x(xmap.rows64, at); at += 64; }
+              if (n_cta & 32) { load_x(xmap.rows32, at); at += 32; }
+              if (n_cta & 16) load_x(xmap.rows16, at);
+            }
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        } else {
+          // scale atoms of this CTA's weight rows and of all the tile's tokens -> this CTA's own barrier
+          // (atoms past the end of the table read as zero and still count their bytes)
+          const int x_atom0 = r.row0 >> 7, x_atoms = ((r.row0 + r.n() - 1) >> 7) - x_atom0 + 1;
+          const int w_atom0 = w_row0 >> 7;
+          const int w_atoms = CTAS == 2 ? 1 : ((w_row0 + w_copy - 1) >> 7) - w_atom0 + 1;
+          const int w_first = (r.expert * p.w_row_atoms + w_atom0) * p.k_blocks, x_first = x_atom0 * p.k_blocks;
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
+            uint8_t* sf = smem + off_sf + stage * L::kSf;
+            if (leader) {
+              mbar_expect_tx(&sf_full[stage], static_cast<uint32_t>(w_atoms + x_atoms) * 512);
+              tma_load_2d(sf, &sfw_map, 0, w_first + kb, &sf_full[stage]);
+              if (L::kSfwAtoms > 1 && w_atoms > 1) tma_load_2d(sf + 512, &sfw_map, 0, w_first + p.k_blocks + kb, &sf_full[stage]);
+              sf += L::kSfwAtoms * 512;
+              tma_load_2d(sf, &sfx_map, 0, x_first + kb, &sf_full[stage]);
+              if (x_atoms > 1) tma_load_2d(sf + 512, &sfx_map, 0, x_first + p.k_blocks + kb, &sf_full[stage]);
+              if (L::kSfxAtoms > 2 && x_atoms > 2)
+                tma_load_2d(sf + 1024, &sfx_map, 0, x_first + 2 * p.k_blocks + kb, &sf_full[stage]);
+            }
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
+          }
         }
       }
       if (!ok) {
         // let copies already in flight land before the CTA retires
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
       }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (even CTA only when paired)
-    if (lane == 0 && cta_rank == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+    } else if (cta_rank == 0) {
+      // ---------------------------------------------------------- MMA issuer (even CTA only when paired)
+      int stage = 0;
+      uint32_t phase = 0;
+      AccCursor cur;
       bool ok = true;
       for (int tile = unit, it = 0; tile < total_tiles && ok; tile += n_units, ++it) {
-        int m_tile, n_tile, e, second, part, rows_lead, rows_peer;
-        if (!fetch_tile(p, sched, tile_table, it, tile, CTAS, m_tile, n_tile, e, second, part, rows_lead, rows_peer))
-          continue;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 2)) break;
+        const TileRec r = fetch_tile<CTAS>(p, sched, tile_table, it, tile);
+        if (r.shape == 0) continue;
+        const bool wide = r.n() > kAccStride;
+        const int acc = cur.begin(wide);
+        if (!mbar_wait(&tmem_empty[acc], (acc ? cur.taken[1] : cur.taken[0]) ^ 1u, abort_flag, p.status, 2)) break;
+        if (wide && !mbar_wait(&tmem_empty[1], cur.taken[1] ^ 1u, abort_flag, p.status, 2)) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BLOCK_N;
-        const int n_row0 = n_tile * BLOCK_N + (part > 0 ? BLOCK_N / 2 : 0);
-        const uint32_t sfb_off = (n_row0 & 127) >> 5;  // a tile may start mid-atom
-        // half tiles run N = 128 MMAs into the first 128 accumulator columns
-        const uint32_t idesc_tile = part >= 0 ? ((idesc_base & ~(0x3Fu << 17)) | (static_cast<uint32_t>(128 >> 3) << 17))
-                                              : idesc_base;
+        const uint32_t d_tmem = tmem_base + acc * kAccStride;
+        const uint32_t idesc_tile = idesc_base | (static_cast<uint32_t>(r.n() >> 3) << 17);
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 3)) { ok = false; break; }
           if constexpr (KIND == 0)
             if (!mbar_wait(&sf_ready[stage], phase, abort_flag, p.status, 5)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sfa_tmem = tmem_base + kSfCol + stage * 16;
-          const uint32_t sfb_tmem = sfa_tmem + 4 + sfb_off;
-          const uint64_t a_desc = desc_sw128(smem_u32(smem + L::kOffA + stage * L::kA));
-          const uint64_t b_desc = desc_sw128(smem_u32(smem + L::kOffB + stage * L::kB));
+          const uint32_t sfw_tmem = tmem_base + kSfCol + stage * kSfSlot;
+          const uint32_t sfx_tmem = sfw_tmem + 4;
+          const uint64_t w_desc = desc_sw128(smem_u32(smem + stage * L::kW));
+          const uint64_t x_desc = desc_sw128(smem_u32(smem + off_x + stage * x_stage));
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if constexpr (KIND == 0) {
-              const uint32_t idesc = idesc_tile | (static_cast<uint32_t>(k) << 29) | (static_cast<uint32_t>(k) << 4);
-              if constexpr (CTAS == 2)
-                tc2_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, sfa_tmem, sfb_tmem, (kb | k) != 0 ? 1u : 0u);
-              else
-                tc_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, sfa_tmem, sfb_tmem, (kb | k) != 0 ? 1u : 0u);
-            } else {
-              if constexpr (CTAS == 2) tc2_mma_bf16(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc_tile, (kb | k) != 0 ? 1u : 0u);
-              else tc_mma_bf16(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc_tile, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
+              if constexpr (KIND == 0) {
+                const uint32_t idesc = idesc_tile | (static_cast<uint32_t>(k) << 29) | (static_cast<uint32_t>(k) << 4);
+                if constexpr (CTAS == 2) tc2_mma_mxf8(d_tmem, w_desc + 2 * k, x_desc + 2 * k, idesc, sfw_tmem, sfx_tmem, accumulate);
+                else tc_mma_mxf8(d_tmem, w_desc + 2 * k, x_desc + 2 * k, idesc, sfw_tmem, sfx_tmem, accumulate);
+              } else {
+                if constexpr (CTAS == 2) tc2_mma_bf16(d_tmem, w_desc + 2 * k, x_desc + 2 * k, idesc_tile, accumulate);
+                else tc_mma_bf16(d_tmem, w_desc + 2 * k, x_desc + 2 * k, idesc_tile, accumulate);
+              }
             }
+            if constexpr (CTAS == 2) tc2_commit_pair(&empty[stage]);
+            else tc_commit(&empty[stage]);
           }
-          if constexpr (CTAS == 2) tc2_commit_pair(&empty[stage]);
-          else tc_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) {
+        if (ok && leader) {
           if constexpr (CTAS == 2) tc2_commit_pair(&tmem_full[acc]);
           else tc_commit(&tmem_full[acc]);
         }
-        if (++acc == kAcc) { acc = 0; acc_phase ^= 1u; }
+        cur.end(wide);
       }
     }
-  }
   } else if (warp < 8) {
     reg_dec<64>();
     // ------------------------------------------------------------ scale-factor movers (one TMEM lane quadrant each)
-    // Lane l of a quadrant owns rows l, l+32, l+64, l+96 of every atom: the 16 bytes at l*16 are the four
-    // 32-bit TMEM cells (4 scale bytes each) the block-scaled MMA expects in that lane.
+    // Row r of an atom sits at byte (r % 32) * 16 + (r / 32) * 4 and belongs in TMEM lane r % 32, column r / 32: for
+    // rows that start on an atom boundary the 16 bytes at lane * 16 are a lane's four columns.  Token rows start at
+    // any multiple of 32 (columns shift), on a single CTA any multiple of 16, like its weight rows (lanes turn too).
     const int q = warp & 3;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = unit, it = 0; KIND == 0 && tile < total_tiles && ok; tile += n_units, ++it) {
-      int m_tile, n_tile, e, second, part, rows_lead, rows_peer;
-      if (!fetch_tile(p, sched, tile_table, it, tile, CTAS, m_tile, n_tile, e, second, part, rows_lead, rows_peer))
-        continue;
+      const TileRec r = fetch_tile<CTAS>(p, sched, tile_table, it, tile);
+      if (r.shape == 0) continue;
+      const int x_off = r.row0 & 127, w_off = CTAS == 2 ? 0 : r.w_row0 & 127;
       for (int kb = 0; kb < p.k_blocks; ++kb) {
         if (!mbar_wait(&sf_full[stage], phase, abort_flag, p.status, 6)) { ok = false; break; }
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kSfCol + stage * 16;
-        {
-          const uint4 va = *reinterpret_cast<const uint4*>(smem + L::kOffSfa + stage * L::kSfa + lane * 16);
-          tc_st4(taddr, va);
+        const uint8_t* sf = smem + off_sf + stage * L::kSf;
+        const uint8_t* sfx = sf + L::kSfwAtoms * 512;
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kSfCol + stage * kSfSlot;
+        auto turned = [&](const uint8_t* atoms, int off, int group) {  // four columns from row off + 32 * group
+          uint32_t v[4];
 #pragma unroll
-          for (int j = 0; j < L::kSfbAtoms; ++j) {
-            const uint4 vb = *reinterpret_cast<const uint4*>(smem + L::kOffSfb + stage * L::kSfb + j * 512 + lane * 16);
-            tc_st4(taddr + 4 + 4 * j, vb);
+          for (int j = 0; j < 4; ++j) {
+            const int row = off + lane + 32 * (group + j);
+            v[j] = *reinterpret_cast<const uint32_t*>(atoms + (row >> 7) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4);
           }
-          tc_wait_st();
+          return make_uint4(v[0], v[1], v[2], v[3]);
+        };
+        if (w_off == 0) tc_st4(taddr, *reinterpret_cast<const uint4*>(sf + lane * 16));
+        else tc_st4(taddr, turned(sf, w_off, 0));
+        if (x_off == 0) {
+          tc_st4(taddr + 4, *reinterpret_cast<const uint4*>(sfx + lane * 16));
+          if constexpr (CTAS == 2) tc_st4(taddr + 8, *reinterpret_cast<const uint4*>(sfx + 512 + lane * 16));
+        } else {
+          tc_st4(taddr + 4, turned(sfx, x_off, 0));
+          if constexpr (CTAS == 2) tc_st4(taddr + 8, turned(sfx, x_off, 4));
         }
+        tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           if (CTAS == 2 && cta_rank != 0) mbar_arrive_leader_relaxed(&sf_ready[stage]);
           else mbar_arrive(&sf_ready[stage]);
         }
-        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else {
     reg_inc<192>();
     // ------------------------------------------------------------ epilogue (every CTA drains its own TMEM)
-    constexpr int kCW = BLOCK_N / 2;   // accumulator columns per thread
-    constexpr int kLd = kCW / 32;      // 32-column TMEM loads per thread
     const int q = warp & 3;
-    const int half = (warp - 8) >> 2;
-    const int row_in_tile = q * 32 + lane;
-    int acc = 0;
-    uint32_t acc_phase = 0;
+    const int group = (warp - 8) >> 2;
+    const int row = q * 32 + lane;  // weight row within this CTA's 128
+    AccCursor cur;
     const bool clamp = (p.gate_lo == p.gate_lo) || (p.gate_hi == p.gate_hi) || (p.up_lo == p.up_lo) ||
                        (p.up_hi == p.up_hi);
-    const float g_lo = p.gate_lo == p.gate_lo ? p.gate_lo : -INFINITY, g_hi = p.gate_hi == p.gate_hi ? p.gate_hi : INFINITY;
-    const float u_lo = p.up_lo == p.up_lo ? p.up_lo : -INFINITY, u_hi = p.up_hi == p.up_hi ? p.up_hi : INFINITY;
+    const float lo_limit = (q & 1) ? p.up_lo : p.gate_lo, hi_limit = (q & 1) ? p.up_hi : p.gate_hi;
+    const float c_lo = lo_limit == lo_limit ? lo_limit : -INFINITY, c_hi = hi_limit == hi_limit ? hi_limit : INFINITY;
+    uint8_t* const group_smem = smem + L::kOffEpi + group * L::kGroup;
+    float* const turn = reinterpret_cast<float*>(group_smem);
+    float* const tok_aff = reinterpret_cast<float*>(group_smem + 2 * kRowBytes);
+    int* const tok_dst = reinterpret_cast<int*>(tok_aff + L::kMaxN / 2);
+    const int tg = threadIdx.x & 127;
+    int out_buf = 0;  // EPI 1: which of the group's two chunk buffers is next
     for (int tile = unit, it = 0; tile < total_tiles; tile += n_units, ++it) {
-      int m_tile, n_tile, e, second, part, rows_lead, rows_peer;
-      if (!fetch_tile(p, sched, tile_table, it, tile, CTAS, m_tile, n_tile, e, second, part, rows_lead, rows_peer))
-        continue;
-      m_tile += cta_rank;
-      if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status, 4)) break;
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BLOCK_N + half * kCW;
-      const int64_t row = static_cast<int64_t>(m_tile) * kBlockM + row_in_tile;
-      uint32_t raw[kLd][32];
+      const TileRec r = fetch_tile<CTAS>(p, sched, tile_table, it, tile);
+      if (r.shape == 0) continue;
+      const int n = r.n();
+      const int w_row0 = r.w_row0 + cta_rank * 128;
+      const int w_rows = min(128, r.w_rows() - cta_rank * 128);  // rows of this CTA that exist (may be <= 0)
+      const int64_t w_index = static_cast<int64_t>(r.expert) * p.n_total + w_row0;
+      // EPI 0: the thread's TMEM lane is its row; EPI 1: rows lane / 4 + 8 i of the warp's 32
+      constexpr int kOwn = EPI == 0 ? 1 : 4;
+      float bias[kOwn], factor[kOwn];
 #pragma unroll
-      for (int l = 0; l < kLd; ++l) tc_ld32_nowait(taddr + l * 32, raw[l]);
+      for (int i = 0; i < kOwn; ++i) {
+        const int own = EPI == 0 ? row : q * 32 + (lane >> 2) + 8 * i;
+        bias[i] = p.bias != nullptr && own < w_rows ? p.bias[w_index + own] : 0.0f;
+        factor[i] = KIND == 1 && p.col_scale != nullptr && own < w_rows ? p.col_scale[w_index + own] : 1.0f;
+      }
+      if constexpr (EPI == 1) {
+        // where each of the group's tokens goes and what it is scaled by, one token per thread, while the MMAs are
+        // still running
+        const int col = (group + 2 * (tg >> 5)) * 32 + lane;
+        if (tg < L::kMaxN / 2) {
+          int dst = -1;
+          float aff = 1.0f;
+          if (col < n) {
+            const int pos = r.row0 + col;
+            const int tok = p.tpi ? p.tpi[pos] : pos;
+            if (tok >= 0 && tok < p.hidden_rows) {
+              dst = pos;
+              if (p.row_src != nullptr) {
+                dst = p.row_src[pos] & 0x7fffffff;
+                if ((dst >> 24) >= 8 || (dst & 0xffffff) >= p.peer_rows || p.peer_out[dst >> 24] == nullptr) dst = -1;
+              }
+              if (p.aff != nullptr)
+                aff = load_as_float(p.aff, p.aff_per_row ? static_cast<int64_t>(tok) : static_cast<int64_t>(tok) * p.E + r.expert,
+                                    p.aff_dtype);
+            }
+          }
+          tok_aff[tg] = aff;
+          tok_dst[tg] = dst;
+        }
+      }
+      const bool wide = n > kAccStride;
+      const int acc = cur.begin(wide);
+      bool ok = mbar_wait(&tmem_full[acc], acc ? cur.filled[1] : cur.filled[0], abort_flag, p.status, 4);
+      ok = group_all(1 + group, ok);  // the group meets at barriers below: leave together
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kAccStride;
+      uint32_t raw[kChunks][32];
+#pragma unroll
+      for (int l = 0; l < kChunks; ++l)
+        if ((group + 2 * l) * 32 < n) {
+          if constexpr (EPI == 0) {
+            tc_ld32_nowait(taddr + (group + 2 * l) * 32, raw[l]);
+          } else {
+            tc_ld16x256_nowait(taddr + (group + 2 * l) * 32, raw[l]);
+            tc_ld16x256_nowait(taddr + (16u << 16) + (group + 2 * l) * 32, raw[l] + 16);
+          }
+        }
       tc_wait_ld();
       // the accumulator now lives in registers: give the TMEM buffer back before doing the math
       tc_fence_before();
@@ -547,131 +751,133 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       if (lane == 0) {
         // relaxed: the accumulator is in registers (wait::ld above); a releasing arrive would first wait for this
         // thread's global stores of the previous tile to become visible and hold the next tile's MMAs back
-        if (CTAS == 2 && cta_rank != 0) mbar_arrive_leader_relaxed(&tmem_empty[acc]);
-        else mbar_arrive_relaxed(&tmem_empty[acc]);
+        for (int a = acc; a <= (wide ? 1 : acc); ++a) {
+          if (CTAS == 2 && cta_rank != 0) mbar_arrive_leader_relaxed(&tmem_empty[a]);
+          else mbar_arrive_relaxed(&tmem_empty[a]);
+        }
       }
-      if (++acc == kAcc) { acc = 0; acc_phase ^= 1u; }
-      if (CTAS == 2 && cta_rank != 0 && !second) continue;  // half-empty pair: these rows belong to someone else
-      if (part >= 0 && half != 0) continue;                 // half tile: only 128 accumulator columns hold results
-      const int n_row0 = n_tile * BLOCK_N + (part > 0 ? BLOCK_N / 2 : 0);
+      cur.end(wide);
+      if (w_rows <= 0) continue;  // uniform across the CTA: the pair's second half lies past the last weight row
 
       if constexpr (EPI == 0) {
-        const int64_t k_atoms = (p.I + 127) >> 7;
-        const float* bias = p.bias ? p.bias + static_cast<int64_t>(e) * p.n_total : nullptr;
+        const int tok_in_chunk = tg >> 2, part = tg & 3;
+        const int blk = part >> 1;  // which 32 intermediates; the thread takes half of them
+        const float* mine = turn + tok_in_chunk * kTurnPitch + blk * 72 + (part & 1) * 16;
+        float* column = turn + row + (q >= 2 ? 8 : 0);
+        const int i0 = (w_row0 >> 1) + blk * 32;
+        const bool have = blk * 64 < w_rows;
 #pragma unroll
-        for (int c = 0; c < kLd / 2; ++c) {
-          const int n0 = n_row0 + half * kCW + c * 64;
-          const int i0 = n0 >> 1;
-          if (i0 >= p.I) continue;
-          float g[32], u[32];
+        for (int l = 0; l < kChunks; ++l) {
+          const int col0 = (group + 2 * l) * 32;
+          if (col0 >= n) break;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) { g[j] = __uint_as_float(raw[2 * c][j]); u[j] = __uint_as_float(raw[2 * c + 1][j]); }
-          if constexpr (KIND == 1) {
-            if (p.col_scale != nullptr) {
-              const float* cs = p.col_scale + static_cast<int64_t>(e) * p.n_total + n0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) { g[j] *= cs[j]; u[j] *= cs[32 + j]; }
-            }
+          for (int j = 0; j < 32; ++j) {
+            float v = __uint_as_float(raw[l][j]);
+            if constexpr (KIND == 1) v *= factor[0];
+            v += bias[0];
+            if (clamp) v = fminf(fmaxf(v, c_lo), c_hi);
+            column[j * kTurnPitch] = v;
           }
-          if (bias != nullptr) {
+          group_barrier(1 + group);
+          float g[16], u[16];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) { g[j] += bias[n0 + j]; u[j] += bias[n0 + 32 + j]; }
+          for (int j = 0; j < 4; ++j) {
+            const float4 a = *reinterpret_cast<const float4*>(mine + 4 * j);
+            const float4 b = *reinterpret_cast<const float4*>(mine + 32 + 4 * j);
+            g[4 * j] = a.x; g[4 * j + 1] = a.y; g[4 * j + 2] = a.z; g[4 * j + 3] = a.w;
+            u[4 * j] = b.x; u[4 * j + 1] = b.y; u[4 * j + 2] = b.z; u[4 * j + 3] = b.w;
           }
-          if (clamp) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              g[j] = fminf(fmaxf(g[j], g_lo), g_hi);
-              u[j] = fminf(fmaxf(u[j], u_lo), u_hi);
-            }
-          }
-          uint32_t mx = 0;
-          if (p.act == B200MOE_ACT_SILU) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float sg = __fdividef(g[j], 1.0f + __expf(-g[j]));
-              const float m = sg * u[j];
-              g[j] = m;
-              mx = max(mx, __float_as_uint(m) & 0x7fffffffu);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float m = apply_act(g[j], p.act) * u[j];
-              g[j] = m;
-              mx = max(mx, __float_as_uint(m) & 0x7fffffffu);
-            }
-          }
+          uint32_t mx = swiglu16(g, u, p.act);
+          const int64_t pos = r.row0 + col0 + tok_in_chunk;
+          const bool store = have && col0 + tok_in_chunk < n;
           if constexpr (KIND == 1) {
             // dense variant: the intermediate stays bf16 (the next contraction's operand type)
-            uint32_t o[16];
+            uint32_t o[8];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < 8; ++j) {
               const __nv_bfloat162 b2 = __floats2bfloat162_rn(g[2 * j], g[2 * j + 1]);
               o[j] = *reinterpret_cast<const uint32_t*>(&b2);
             }
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.m_codes) + row * p.I + i0;
-            st_global_256(dst, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]);
-            st_global_256(dst + 16, o[8], o[9], o[10], o[11], o[12], o[13], o[14], o[15]);
-            continue;
-          }
-          uint32_t w[8];
-          const int e_max = static_cast<int>(mx >> 23);
-          if (e_max >= 9) {  // one exact power-of-two factor
-            const float f = __uint_as_float(static_cast<uint32_t>(135 - e_max + 127) << 23);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) w[j] = pack4_e4m3(g[4 * j] * f, g[4 * j + 1] * f, g[4 * j + 2] * f, g[4 * j + 3] * f);
+            if (store)
+              st_global_256(reinterpret_cast<__nv_bfloat16*>(p.m_codes) + pos * p.I + i0 + (part & 1) * 16, o[0], o[1], o[2],
+                            o[3], o[4], o[5], o[6], o[7]);
           } else {
-            float f1, f2;
-            mx_block_factors(mx, f1, f2);
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            uint32_t w[4];
+            const int e_max = static_cast<int>(mx >> 23);
+            if (e_max >= 9) {  // one exact power-of-two factor
+              const float f = __uint_as_float(static_cast<uint32_t>(135 - e_max + 127) << 23);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              w[j] = pack4_e4m3(g[4 * j] * f1 * f2, g[4 * j + 1] * f1 * f2, g[4 * j + 2] * f1 * f2, g[4 * j + 3] * f1 * f2);
+              for (int j = 0; j < 4; ++j) w[j] = pack4_e4m3(g[4 * j] * f, g[4 * j + 1] * f, g[4 * j + 2] * f, g[4 * j + 3] * f);
+            } else {
+              float f1, f2;
+              mx_block_factors(mx, f1, f2);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                w[j] = pack4_e4m3(g[4 * j] * f1 * f2, g[4 * j + 1] * f1 * f2, g[4 * j + 2] * f1 * f2, g[4 * j + 3] * f1 * f2);
+            }
+            if (store) {
+              *reinterpret_cast<uint4*>(p.m_codes + pos * p.I + i0 + (part & 1) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+              if ((part & 1) == 0) p.m_sf[sf_atom_offset(pos, i0 >> 5, (p.I + 127) >> 7)] = mx_block_scale_byte(mx);
+            }
           }
-          st_global_256(p.m_codes + row * p.I + i0, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7]);
-          p.m_sf[sf_atom_offset(row, i0 >> 5, k_atoms)] = mx_block_scale_byte(mx);
+          group_barrier(1 + group);  // the chunk buffer is free again
         }
       } else {
-        const int tok = p.tpi ? p.tpi[row] : static_cast<int>(row);
-        bool valid = tok >= 0 && tok < p.hidden_rows;
-        __nv_bfloat16* out_row = p.y_pos + row * p.H_out;
-        if (p.row_src != nullptr && valid) {
-          const int32_t src = p.row_src[row];
-          const int dst_rank = (src >> 24) & 0x7f;
-          const int64_t dst_row = src & 0xffffff;
-          valid = dst_rank < 8 && dst_row < p.peer_rows && p.peer_out[dst_rank] != nullptr;
-          if (valid) out_row = static_cast<__nv_bfloat16*>(p.peer_out[dst_rank]) + dst_row * p.H_out;
-        }
-        float aff = 1.0f;
-        if (valid && p.aff != nullptr)
-          aff = load_as_float(p.aff, p.aff_per_row ? static_cast<int64_t>(tok) : static_cast<int64_t>(tok) * p.E + e,
-                              p.aff_dtype);
-        const float* bias = p.bias ? p.bias + static_cast<int64_t>(e) * p.H_out : nullptr;
-        const float* cs = (KIND == 1 && p.col_scale) ? p.col_scale + static_cast<int64_t>(e) * p.H_out : nullptr;
+        // A thread holds, of every 8 tokens, tokens 2 (lane % 4) and + 1 of four weight rows (lane / 4 + 8 i): packed to
+        // bf16 pairs these are the fragments of four 8 x 8 matrices, which the transposing matrix store turns into
+        // 16-byte pieces of token rows.  A bulk copy per token then moves 256 contiguous bytes to global memory: the
+        // stores cost no registers and no L1 write slots (with 4-byte stores from registers the short contractions
+        // ran at half the speed).
+        const float2* const aff2 = reinterpret_cast<const float2*>(tok_aff) + (lane & 3);
+        const uint32_t row_bytes = static_cast<uint32_t>(w_rows) * 2;
 #pragma unroll
-        for (int l = 0; l < kLd; ++l) {
-          const int col0 = n_row0 + half * kCW + l * 32;
-          if (col0 >= p.H_out || !valid) continue;
-          uint32_t o[16];
+        for (int l = 0; l < kChunks; ++l) {
+          if ((group + 2 * l) * 32 >= n) break;
+          uint8_t* const buf = group_smem + out_buf * kRowBytes;
+          out_buf ^= 1;
+          // the copies out of this buffer two chunks ago (issued by lanes of these warps) have read it
+          asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          group_barrier(1 + group);
+          const uint32_t to = smem_u32(buf) + (lane & 7) * kRowPitch + (q * 32 + (lane >> 3) * 8) * 2;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float a0 = __uint_as_float(raw[l][2 * j]), a1 = __uint_as_float(raw[l][2 * j + 1]);
-            if (cs) { a0 *= cs[col0 + 2 * j]; a1 *= cs[col0 + 2 * j + 1]; }
-            if (bias) { a0 += bias[col0 + 2 * j]; a1 += bias[col0 + 2 * j + 1]; }
-            const __nv_bfloat162 b2 = __floats2bfloat162_rn(a0 * aff, a1 * aff);
-            o[j] = *reinterpret_cast<const uint32_t*>(&b2);
+          for (int g = 0; g < 4; ++g) {
+            const float2 a = aff2[l * 16 + g * 4];
+            uint32_t m[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float v0 = __uint_as_float(raw[l][(i >> 1) * 16 + g * 4 + (i & 1) * 2]);
+              float v1 = __uint_as_float(raw[l][(i >> 1) * 16 + g * 4 + (i & 1) * 2 + 1]);
+              if constexpr (KIND == 1) { v0 *= factor[i]; v1 *= factor[i]; }
+              const __nv_bfloat162 b2 = __floats2bfloat162_rn((v0 + bias[i]) * a.x, (v1 + bias[i]) * a.y);
+              m[i] = *reinterpret_cast<const uint32_t*>(&b2);
+            }
+            stmatrix_x4_trans(to + g * 8 * kRowPitch, m[0], m[1], m[2], m[3]);
           }
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            st_global_256(out_row + col0 + 16 * j, o[8 * j], o[8 * j + 1], o[8 * j + 2], o[8 * j + 3], o[8 * j + 4],
-                          o[8 * j + 5], o[8 * j + 6], o[8 * j + 7]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          group_barrier(1 + group);
+          const int c = q * 8 + (lane & 7);
+          const int dst = tok_dst[l * 32 + c];
+          if (p.row_src == nullptr) {
+            if (lane < 8 && dst >= 0)
+              bulk_store(p.y_pos + static_cast<int64_t>(dst) * p.H_out + w_row0, buf + c * kRowPitch, row_bytes);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          } else if (dst >= 0) {
+            // to the GPU the token came from: four lanes per row, 16 bytes each at a time
+            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.peer_out[dst >> 24]) +
+                                 static_cast<int64_t>(dst & 0xffffff) * p.H_out + w_row0;
+            for (int b = (lane >> 3) * 8; b < w_rows; b += 32)
+              *reinterpret_cast<uint4*>(out + b) = *reinterpret_cast<const uint4*>(buf + c * kRowPitch + b * 2);
+          }
         }
+        // the token list may change once every thread of the group is past its reads of it
+        group_barrier(1 + group);
       }
     }
+    // copies read this CTA's shared memory and must be complete before the grid is
+    if constexpr (EPI == 1) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
-  // A grid that was allowed to start while its predecessor drains must not finish before it: whatever follows in
-  // the stream waits for this grid only, and relies on both having completed.
-  if (p.wait_predecessor) asm volatile("griddepcontrol.wait;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   if (p.clock_probe != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -751,14 +957,14 @@ __global__ void simt_gemm1_kernel(const uint8_t* x, const uint8_t* w, GemmParams
     const int e = p.block_to_expert[block];
     if (e < 0 || e >= p.E) continue;
     const uint8_t* we = w + weight_offset(static_cast<int64_t>(e) * p.n_total, K, p.w_format);
-    const uint8_t* wsf = p.b_sf + static_cast<int64_t>(e) * p.b_sf_expert_stride;
+    const uint8_t* wsf = p.w_sf + static_cast<int64_t>(e) * p.w_sf_expert_stride;
     const float* bias = p.bias ? p.bias + static_cast<int64_t>(e) * p.n_total : nullptr;
     float m[32];
     uint32_t mx = 0;
     for (int j = 0; j < 32; ++j) {
       const int n_g = ib * 64 + j, n_u = n_g + 32;
-      float gv = mx_dot(x, p.a_sf, row, we, wsf, n_g, K, p.w_format);
-      float uv = mx_dot(x, p.a_sf, row, we, wsf, n_u, K, p.w_format);
+      float gv = mx_dot(x, p.x_sf, row, we, wsf, n_g, K, p.w_format);
+      float uv = mx_dot(x, p.x_sf, row, we, wsf, n_u, K, p.w_format);
       if (bias) { gv += bias[n_g]; uv += bias[n_u]; }
       if (p.gate_lo == p.gate_lo) gv = fmaxf(gv, p.gate_lo);
       if (p.gate_hi == p.gate_hi) gv = fminf(gv, p.gate_hi);
@@ -790,8 +996,8 @@ __global__ void simt_gemm2_kernel(const uint8_t* m, const uint8_t* w, GemmParams
     if (e < 0 || e >= p.E) continue;
     const int tok = p.tpi ? p.tpi[row] : static_cast<int>(row);
     if (tok < 0 || tok >= p.hidden_rows) continue;
-    float y = mx_dot(m, p.a_sf, row, w + weight_offset(static_cast<int64_t>(e) * p.n_total, K, p.w_format),
-                     p.b_sf + static_cast<int64_t>(e) * p.b_sf_expert_stride, h, K, p.w_format);
+    float y = mx_dot(m, p.x_sf, row, w + weight_offset(static_cast<int64_t>(e) * p.n_total, K, p.w_format),
+                     p.w_sf + static_cast<int64_t>(e) * p.w_sf_expert_stride, h, K, p.w_format);
     if (p.bias) y += p.bias[static_cast<int64_t>(e) * p.H_out + h];
     if (p.aff)
       y *= load_as_float(p.aff, p.aff_per_row ? static_cast<int64_t>(tok) : static_cast<int64_t>(tok) * p.E + e,
@@ -906,55 +1112,38 @@ int make_atoms_map(CUtensorMap* map, const void* base, int64_t n_atoms) {
   return B200MOE_OK;
 }
 
-template <int BLOCK_N, int STAGES, int EPI, int CTAS, int KIND = 0>
-int launch_tc(const CUtensorMap (&ma)[3], const CUtensorMap& mb, const CUtensorMap& mb128, const CUtensorMap& msa,
-              const CUtensorMap& msb, const GemmParams& p, cudaStream_t st, bool overlap_predecessor = false) {
-  using L = SmemLayout<BLOCK_N, STAGES, CTAS>;
-  auto kern = grouped_mxfp8_gemm_kernel<BLOCK_N, STAGES, EPI, CTAS, KIND>;
+template <int EPI, int CTAS, int KIND>
+int launch_tc(const WeightMaps& wm, const TokenMaps& xm, const CUtensorMap& sfw, const CUtensorMap& sfx,
+              const GemmParams& p, cudaStream_t st) {
+  using L = SmemLayout<EPI, CTAS>;
+  auto kern = grouped_mxfp8_gemm_kernel<EPI, CTAS, KIND>;
+  static_assert(L::kBytes <= 227 * 1024, "shared memory of the contraction kernel");
   B200MOE_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kBytes));
-  // only sizes the grid; a left-over launch has at most one tile per expert and weight tile
-  const int total = p.tile_filter == 2 ? p.E * p.n_tiles : ((p.m_tiles_total + CTAS - 1) / CTAS) * p.n_tiles;
-  int grid = (total < sm_count() / CTAS ? total : sm_count() / CTAS) * CTAS;
-  if constexpr (CTAS == 2) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = L::kBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    B200MOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma[0], ma[1], ma[2], mb, mb128, msa, msb, p));
-  } else if (overlap_predecessor) {
-    // programmatic stream serialisation: this grid may be scheduled while the previous kernel of the stream is
-    // still draining (the kernel never waits for it: it shares no rows with it)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = L::kBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    B200MOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma[0], ma[1], ma[2], mb, mb128, msa, msb, p));
-  } else {
-    kern<<<grid, kThreads, L::kBytes, st>>>(ma[0], ma[1], ma[2], mb, mb128, msa, msb, p);
-  }
+  // only sizes the grid: at most one token tile per 128 positions; a single CTA may cut its 128 weight rows further
+  const int64_t total = static_cast<int64_t>(p.m_tiles_total) * ceil_div64(p.n_total, CTAS == 2 ? 256 : (EPI == 0 ? 64 : 16));
+  const int units = sm_count() / CTAS;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((total < units ? total : units) * CTAS));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::kBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CTAS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CTAS == 2 ? 1 : 0;
+  B200MOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, wm, xm, sfw, sfx, p));
   B200MOE_LAUNCH_OK("grouped_mxfp8_gemm_kernel");
   return B200MOE_OK;
 }
 
 // `impl` is the per-call variant word of the entry points: bit 0 selects the CUDA-core validation kernels, the
 // B200MOE_GEMM_* bits restrict the tile shapes the tensor-core path may pick.  Nothing here is process state.
-// `kind`: 0 = MX (a and b are element codes, K counts elements = bytes, or nibbles for e2m1 weights); 1 = dense
+// `kind`: 0 = MX (x and w are element codes, K counts elements = bytes, or nibbles for e2m1 weights); 1 = dense
 // bf16 operands (K counts bf16 elements; the copies address rows in bytes).
-int run_gemm(int epi, const uint8_t* a, const uint8_t* b, GemmParams& p, int K, int impl, void* clock_probe,
+int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, int impl, void* clock_probe,
              cudaStream_t st, int kind = 0) {
   B200MOE_REQUIRE((impl & ~(B200MOE_IMPL_SIMT | B200MOE_GEMM_TILE_N128 | B200MOE_GEMM_NO_PAIR | B200MOE_GEMM_FORCE_PAIR |
                             B200MOE_GEMM_NO_SPLIT | B200MOE_GEMM_NO_OVERLAP)) == 0,
@@ -977,8 +1166,8 @@ int run_gemm(int epi, const uint8_t* a, const uint8_t* b, GemmParams& p, int K, 
   p.clock_probe = static_cast<unsigned long long*>(clock_probe);
   const int Kb = kind == 1 ? 2 * K : K;  // row pitch the copies see, in element-code bytes
   p.k_blocks = (Kb + kBlockK - 1) / kBlockK;
-  p.b_row_atoms = (p.n_total + 127) / 128;
-  p.b_sf_expert_stride = static_cast<int64_t>(p.b_row_atoms) * p.k_blocks * 512;
+  p.w_row_atoms = (p.n_total + 127) / 128;
+  p.w_sf_expert_stride = static_cast<int64_t>(p.w_row_atoms) * p.k_blocks * 512;
   B200MOE_CUDA_OK(cudaMemsetAsync(p.status, 0, 4, st));
   if (impl & B200MOE_IMPL_SIMT) {
     const int64_t work = epi == 0 ? static_cast<int64_t>(p.m_tiles_total) * 128 * (p.I / 32)
@@ -986,78 +1175,49 @@ int run_gemm(int epi, const uint8_t* a, const uint8_t* b, GemmParams& p, int K, 
     const int64_t cap = static_cast<int64_t>(sm_count()) * 32;
     const int grid = static_cast<int>(ceil_div64(work, 128) < cap ? ceil_div64(work, 128) : cap);
     if (kind == 1) {
-      const auto* ab = reinterpret_cast<const __nv_bfloat16*>(a);
-      const auto* bb = reinterpret_cast<const __nv_bfloat16*>(b);
+      const auto* ab = reinterpret_cast<const __nv_bfloat16*>(x);
+      const auto* bb = reinterpret_cast<const __nv_bfloat16*>(w);
       if (epi == 0) simt_dense_gemm1_kernel<<<grid, 128, 0, st>>>(ab, bb, p, K);
       else simt_dense_gemm2_kernel<<<grid, 128, 0, st>>>(ab, bb, p, K);
-    } else if (epi == 0) simt_gemm1_kernel<<<grid, 128, 0, st>>>(a, b, p, K);
-    else simt_gemm2_kernel<<<grid, 128, 0, st>>>(a, b, p, K);
+    } else if (epi == 0) simt_gemm1_kernel<<<grid, 128, 0, st>>>(x, w, p, K);
+    else simt_gemm2_kernel<<<grid, 128, 0, st>>>(x, w, p, K);
     B200MOE_LAUNCH_OK("simt_gemm_kernel");
     return B200MOE_OK;
   }
-  B200MOE_REQUIRE(K % 16 == 0, B200MOE_ERR_INVALID, "TMA needs row pitches that are multiples of 16 bytes");
-  const int bn = (impl & B200MOE_GEMM_TILE_N128) ? 128 : 256;
-  const bool split_leftover = !(impl & B200MOE_GEMM_NO_SPLIT);
-  const bool overlap_leftover = !(impl & B200MOE_GEMM_NO_OVERLAP);
-  p.n_tiles = (p.n_total + bn - 1) / bn;
-  // CTA pairs need two position tiles per weight tile: always there when a block holds an even number of 128-row
-  // tiles; with odd blocks (B = 128) an expert's tiles are paired across its blocks, which pays once experts have
-  // several tiles on average (prefill) and not for one short tile per expert (decode)
-  const bool pair = !(impl & B200MOE_GEMM_NO_PAIR) && bn == 256 && (sm_count() % 2 == 0) &&
-                    (p.B % 256 == 0 || (impl & B200MOE_GEMM_FORCE_PAIR) || p.m_tiles_total >= 4 * p.E);
-  CUtensorMap ma[3], mb, mb128, msa, msb;  // activation boxes of 128, 64 and 32 rows; weight boxes: tile, 128 rows
-  int rc = B200MOE_OK;
-  for (int i = 0; i < 3 && rc == B200MOE_OK; ++i)
-    rc = make_rows_map(&ma[i], a, Kb, static_cast<int64_t>(p.m_tiles_total) * 128, 0, kBlockM >> i);
-  if (rc != B200MOE_OK) return rc;
-  rc = make_rows_map(&mb, b, Kb, p.n_total, p.E, pair ? bn / 2 : bn, nibbles);
-  // the copy reports the bytes it read from global memory: a 4-bit slab is 64 bytes per row there
-  p.b_tx = static_cast<uint32_t>((pair ? bn / 2 : bn) * (nibbles ? kBlockK / 2 : kBlockK));
-  if (rc != B200MOE_OK) return rc;
-  rc = make_rows_map(&mb128, b, Kb, p.n_total, p.E, 128, nibbles);  // half tiles of the single-CTA launches
-  if (rc != B200MOE_OK) return rc;
-  if (kind == 0) {
-    rc = make_atoms_map(&msa, p.a_sf, static_cast<int64_t>(p.m_tiles_total) * p.k_blocks);
+  // CTA pairs (256 weight rows, up to 256 tokens per tile) once experts can hold more than one 128-row tile on average:
+  // each CTA then copies half of the token rows.  Below that a launch is bound by streaming the weights, and single CTAs
+  // (128 weight rows or fewer) spread the rows over the SMs in finer pieces.  Tiles of up to 256 tokens although only
+  // 224 leave room for a second accumulator: the 8192-token layer above took 4.2 ms with tiles of at most 224 and 3.9
+  // with 256, the 4096-token one 1.244 and 1.233 -- fewer operand bytes per MMA outweigh the drain at a tile's end.
+  const bool pair = !(impl & (B200MOE_GEMM_NO_PAIR | B200MOE_GEMM_TILE_N128)) && (sm_count() % 2 == 0) &&
+                    (p.B % 256 == 0 || (impl & B200MOE_GEMM_FORCE_PAIR) || p.m_tiles_total >= 2 * p.E);
+  p.max_n = pair ? 256 : 128;
+  p.w_slab_bytes = nibbles ? kBlockK / 2 : kBlockK;
+  WeightMaps wm;
+  TokenMaps xm;
+  CUtensorMap* const w_maps[4] = {&wm.rows128, &wm.rows64, &wm.rows32, &wm.rows16};
+  CUtensorMap* const x_maps[4] = {&xm.rows128, &xm.rows64, &xm.rows32, &xm.rows16};
+  CUtensorMap sfx, sfw;
+  for (int i = 0; i < 4; ++i) {
+    int rc = make_rows_map(x_maps[i], x, Kb, static_cast<int64_t>(p.m_tiles_total) * 128, 0, 128 >> i);
     if (rc != B200MOE_OK) return rc;
-    rc = make_atoms_map(&msb, p.b_sf, static_cast<int64_t>(p.E) * p.b_row_atoms * p.k_blocks);
+    rc = make_rows_map(w_maps[i], w, Kb, p.n_total, p.E, 128 >> i, nibbles);
+    if (rc != B200MOE_OK) return rc;
+  }
+  if (kind == 0) {
+    int rc = make_atoms_map(&sfx, p.x_sf, static_cast<int64_t>(p.m_tiles_total) * p.k_blocks);
+    if (rc != B200MOE_OK) return rc;
+    rc = make_atoms_map(&sfw, p.w_sf, static_cast<int64_t>(p.E) * p.w_row_atoms * p.k_blocks);
     if (rc != B200MOE_OK) return rc;
   } else {
-    msa = msb = ma[0];  // never dereferenced by the dense kernel
+    sfx = sfw = xm.rows128;  // never dereferenced by the dense kernel
   }
   if (pair) {
-    // Two launches: the CTA-pair kernel walks the pairs of live 128-row tiles, the single-CTA kernel the one
-    // tile an expert with an odd number of live tiles has left over (a half-empty pair would pay for a full
-    // 256-row MMA: with ~1000 rows per expert that was one tile in five).
-    p.tile_filter = split_leftover ? 1 : 0;
-    p.early_successor = (split_leftover && overlap_leftover) ? 1 : 0;
-    if (kind == 1)
-      rc = epi == 0 ? launch_tc<256, 6, 0, 2, 1>(ma, mb, mb128, msa, msb, p, st)
-                    : launch_tc<256, 6, 1, 2, 1>(ma, mb, mb128, msa, msb, p, st);
-    else
-      rc = epi == 0 ? launch_tc<256, 6, 0, 2>(ma, mb, mb128, msa, msb, p, st) : launch_tc<256, 6, 1, 2>(ma, mb, mb128, msa, msb, p, st);
-    if (rc != B200MOE_OK || !split_leftover) return rc;
-    GemmParams p2 = p;
-    p2.tile_filter = 2;
-    p2.early_successor = 0;
-    p2.wait_predecessor = overlap_leftover ? 1 : 0;
-    p2.clock_probe = nullptr;
-    p2.b_tx = static_cast<uint32_t>(bn * (nibbles ? kBlockK / 2 : kBlockK));
-    CUtensorMap mb2;
-    rc = make_rows_map(&mb2, b, Kb, p.n_total, p.E, bn, nibbles);
-    if (rc != B200MOE_OK) return rc;
-    const bool ov = overlap_leftover;
-    if (kind == 1)
-      return epi == 0 ? launch_tc<256, 4, 0, 1, 1>(ma, mb2, mb128, msa, msb, p2, st, ov)
-                      : launch_tc<256, 4, 1, 1, 1>(ma, mb2, mb128, msa, msb, p2, st, ov);
-    return epi == 0 ? launch_tc<256, 4, 0, 1>(ma, mb2, mb128, msa, msb, p2, st, ov)
-                    : launch_tc<256, 4, 1, 1>(ma, mb2, mb128, msa, msb, p2, st, ov);
+    if (kind == 1) return epi == 0 ? launch_tc<0, 2, 1>(wm, xm, sfw, sfx, p, st) : launch_tc<1, 2, 1>(wm, xm, sfw, sfx, p, st);
+    return epi == 0 ? launch_tc<0, 2, 0>(wm, xm, sfw, sfx, p, st) : launch_tc<1, 2, 0>(wm, xm, sfw, sfx, p, st);
   }
-  if (kind == 1)
-    return epi == 0 ? launch_tc<256, 4, 0, 1, 1>(ma, mb, mb128, msa, msb, p, st)
-                    : launch_tc<256, 4, 1, 1, 1>(ma, mb, mb128, msa, msb, p, st);
-  if (bn == 256)
-    return epi == 0 ? launch_tc<256, 4, 0, 1>(ma, mb, mb128, msa, msb, p, st) : launch_tc<256, 4, 1, 1>(ma, mb, mb128, msa, msb, p, st);
-  return epi == 0 ? launch_tc<128, 6, 0, 1>(ma, mb, mb128, msa, msb, p, st) : launch_tc<128, 6, 1, 1>(ma, mb, mb128, msa, msb, p, st);
+  if (kind == 1) return epi == 0 ? launch_tc<0, 1, 1>(wm, xm, sfw, sfx, p, st) : launch_tc<1, 1, 1>(wm, xm, sfw, sfx, p, st);
+  return epi == 0 ? launch_tc<0, 1, 0>(wm, xm, sfw, sfx, p, st) : launch_tc<1, 1, 0>(wm, xm, sfw, sfx, p, st);
 }
 
 }  // namespace
@@ -1079,8 +1239,8 @@ extern "C" int b200moe_grouped_gemm1_swiglu(const uint8_t* x_codes, const uint8_
   B200MOE_REQUIRE((reinterpret_cast<uintptr_t>(m_codes) & 31) == 0, B200MOE_ERR_INVALID,
                   "grouped_gemm1: m_codes must be 32-byte aligned (the epilogue stores 32 bytes at a time)");
   GemmParams p{};
-  p.a_sf = x_sf;
-  p.b_sf = w1_sf;
+  p.x_sf = x_sf;
+  p.w_sf = w1_sf;
   p.w_format = w_format;
   p.block_to_expert = block_to_expert;
   p.conditions = conditions;
@@ -1118,8 +1278,8 @@ int gemm2_impl(const uint8_t* m_codes, const uint8_t* m_sf, const uint8_t* w2_de
   B200MOE_REQUIRE(aff_dtype == B200MOE_F32 || aff_dtype == B200MOE_BF16, B200MOE_ERR_INVALID,
                   "grouped_gemm2: affinities must be fp32 or bf16");
   GemmParams p{};
-  p.a_sf = m_sf;
-  p.b_sf = w2_sf;
+  p.x_sf = m_sf;
+  p.w_sf = w2_sf;
   p.w_format = w_format;
   p.block_to_expert = block_to_expert;
   p.conditions = conditions;

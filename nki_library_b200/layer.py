@@ -3,7 +3,7 @@
 This is the call sequence the reference leaves to its caller for prefill
 (router and grouping sub-kernels, then ``moe_cte``) and fuses for decode in
 ``moe_block_tkg`` (core/moe_block/moe_block_tkg.py:192-340, without the RMSNorm).
-All buffers are allocated once; a forward pass launches nine to twelve kernels
+All buffers are allocated once; a forward pass launches seven to ten kernels
 (``kernels_per_forward``) on the current stream and never synchronises with the
 host.
 """
@@ -55,14 +55,12 @@ class MoELayer:
         self.ws = pipeline.BlockWorkspace(self.N * B, self.H, self.I, dev)
         self.out = torch.empty((T, self.H), dtype=torch.bfloat16, device=dev)
         # launches per forward pass: router (logits + ranking, or weight transpose + tcgen05 logits + ranking for
-        # large T), grouping (3, or 1 up to 256 tokens), quantise, the contractions (CTA-pair launch + left-over launch each when the
-        # library takes its pair path, else one each), combine -- mirrors the library's own shape rules
+        # large T), grouping (3, or 1 up to 256 tokens), quantise, the two contractions, combine -- mirrors the
+        # library's own shape rules
         tc_ok = E <= 256 and self.H % 64 == 0
         router_launches = 3 if (tc_ok and (router_path == 2 or (router_path == 0 and T >= 8192))) else 2
-        pair_path = not (gemm_variant & (_lib.GEMM_NO_PAIR | _lib.GEMM_TILE_N128)) and (
-            B % 256 == 0 or bool(gemm_variant & _lib.GEMM_FORCE_PAIR) or self.N * (B // 128) >= 4 * E)
         group_launches = 1 if T <= 256 else 3  # one 256-token chunk: the three grouping phases share a CTA
-        self.kernels_per_forward = router_launches + group_launches + 1 + (2 if not pair_path else (2 if gemm_variant & _lib.GEMM_NO_SPLIT else 4)) + 1
+        self.kernels_per_forward = router_launches + group_launches + 1 + 2 + 1
 
     def forward(self, hidden: torch.Tensor, timers: Optional[dict] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:

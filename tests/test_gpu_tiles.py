@@ -1,0 +1,57 @@
+"""Tile edges of the grouped contraction kernel: token counts around its tile widths, weight rows that fill no whole
+tile, blocks with holes.  The tensor-core path against the CUDA-core kernels on the same quantised inputs.
+
+Tolerance, as max|a - b| / max|b|: both sides round each output to bf16 (half a step each, together 2^-8), and where an
+intermediate lies on a rounding tie of its e4m3 code the two summation orders may take different sides, which moves an
+output by 2^-4 of one of its I >= 32 terms; 1e-2 covers both with a factor of two."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-2
+
+
+def _blocks(counts, B, holes):
+    """token_position_to_id / block_to_expert for ``counts[e]`` tokens of expert e, ids in order of position; with
+    ``holes`` the first block of an expert that has several is left half empty."""
+    tpi, b2e, t = [], [], 0
+    for e, n in enumerate(counts):
+        left = n
+        while left > 0:
+            take = min(left, B // 2 - 3 if holes and left == n and n > B else B)
+            tpi += list(range(t, t + take)) + [-1] * (B - take)
+            b2e.append(e)
+            t, left = t + take, left - take
+    i32 = dict(dtype=torch.int32, device="cuda")
+    return torch.tensor(tpi, **i32), torch.tensor(b2e, **i32), t
+
+
+@pytest.mark.parametrize("variant", ["single", "pair"])
+@pytest.mark.parametrize("counts,B,H,I,holes", [
+    ([1, 15, 16, 17, 0, 31, 33], 128, 256, 32, False),
+    ([127, 128, 129, 255], 128, 128, 96, False),
+    ([223, 224, 225, 1], 256, 160, 416, False),
+    ([256, 257, 448, 449, 513], 256, 128, 160, False),
+    ([700, 3, 300], 128, 256, 64, True),
+])
+def test_tile_edges(variant, counts, B, H, I, holes):
+    import nki_library_b200 as m
+    from nki_library_b200 import _lib
+    from nki_library_b200.layer import random_expert_weights
+    tpi, b2e, T = _blocks(counts, B, holes)
+    E = len(counts)
+    g = torch.Generator(device="cuda").manual_seed(T + I)
+    w = random_expert_weights(E, H, I, "cuda", seed=I)
+    w.bias_gu = torch.randn((E, 2 * I), device="cuda", generator=g) * 0.5
+    w.bias_d = torch.randn((E, H), device="cuda", generator=g) * 0.5
+    x = torch.randn((T, H), device="cuda", generator=g).to(torch.bfloat16)
+    aff = torch.rand((T, E), device="cuda", generator=g)
+
+    def run(impl):
+        return m.moe_cte(x, aff.view(-1, 1), w, None, tpi, b2e, B, m.MoECTESpec(m.MoECTEImplementation.shard_on_block_mx),
+                         skip_dma=m.SkipMode(True, False), _impl=impl, _check_status=True).float()
+
+    ref = run(_lib.IMPL_SIMT)
+    got = run(_lib.GEMM_NO_PAIR if variant == "single" else _lib.GEMM_FORCE_PAIR)
+    assert float((got - ref).abs().max() / ref.abs().max()) <= TOL
