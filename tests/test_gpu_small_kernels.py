@@ -1,0 +1,103 @@
+"""The bookkeeping and row kernels around the contractions at the edges of their loops: position lists longer than one
+round, columns past a whole number of vectors, more chunks than one thread scans.  Integer results and copies are
+compared exactly; the RMSNorm against fp64 torch within one bf16 rounding (2^-8 of the value) and the combine with the
+fp32 sum in the same order."""
+
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _lib():
+    from nki_library_b200 import _lib
+    return _lib
+
+
+def _gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _positions(T, K, n_pos, share, seed):
+    """[T, K] table of distinct positions, a share of the entries empty, some of those out of range."""
+    g = _gen(seed)
+    table = torch.randperm(n_pos, device="cuda", generator=g)[:T * K].reshape(T, K).to(torch.int32)
+    drop = torch.rand((T, K), device="cuda", generator=g) >= share
+    return torch.where(drop, torch.where(torch.arange(K, device="cuda") % 2 == 0, -1, n_pos + 5).to(torch.int32), table)
+
+
+@pytest.mark.parametrize("T,H,K,share", [(3, 512, 1, 1.0), (9, 1024, 8, 1.0), (17, 1152, 33, 0.3), (5, 2176, 129, 0.1),
+                                         (2, 3072, 300, 0.5)])
+@pytest.mark.parametrize("packed", [0, 1])
+def test_scatter_quantize_long_lists(T, H, K, share, packed):
+    L = _lib()
+    H = (H + 511) // 512 * 512 if packed else H
+    n_pos = (T * K + 127) // 128 * 128
+    table = _positions(T, K, n_pos, share, H + K)
+    x = torch.randn((T, H), device="cuda", generator=_gen(1)).to(torch.bfloat16)
+    nsf = L.load_library().b200moe_sf_bytes(n_pos, H)
+
+    def buffers():
+        return (torch.zeros((n_pos, H), dtype=torch.uint8, device="cuda"), torch.zeros(nsf, dtype=torch.uint8, device="cuda"),
+                torch.zeros((n_pos // 128,), dtype=torch.int32, device="cuda"))
+
+    got = buffers()
+    L.call("b200moe_scatter_quantize_mxfp8", L.ptr(x), T, H, L.ptr(table), K, n_pos, packed, *map(L.ptr, got), L.stream_ptr())
+    # the position-major kernel on the forward map of the same table
+    tpi = torch.full((n_pos,), -1, dtype=torch.int32, device="cuda")
+    ok = (table >= 0) & (table < n_pos)
+    tpi[table[ok].long()] = torch.arange(T, dtype=torch.int32, device="cuda")[:, None].expand(T, K)[ok]
+    ref = buffers()
+    L.call("b200moe_gather_quantize_mxfp8", L.ptr(x), T, H, L.ptr(tpi), n_pos, packed, *map(L.ptr, ref), L.stream_ptr())
+    held = tpi >= 0
+    assert torch.equal(got[0][held], ref[0][held]) and torch.equal(got[2], ref[2])
+    pos = torch.arange(n_pos, device="cuda")
+    kb = torch.arange(H // 32, device="cuda")
+    at = (((pos >> 7)[:, None] * ((H + 127) // 128) + (kb >> 2)[None]) * 512 + (pos & 31)[:, None] * 16 +
+          (((pos >> 5) & 3) * 4)[:, None] + (kb & 3)[None])
+    assert torch.equal(got[1][at][held], ref[1][at][held])
+
+
+@pytest.mark.parametrize("T,H,K", [(1, 8, 1), (7, 1032, 3), (11, 4104, 130)])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_scatter_rows(T, H, K, scaled):
+    L = _lib()
+    B, E = 128, 5
+    n_pos = (T * K + B - 1) // B * B
+    table = _positions(T, K, n_pos, 0.6, H)
+    x = torch.randn((T, H), device="cuda", generator=_gen(2)).to(torch.bfloat16)
+    b2e = torch.randint(0, E, (n_pos // B,), dtype=torch.int32, device="cuda", generator=_gen(3))
+    aff = torch.rand((T, E), device="cuda", generator=_gen(4))
+    out = torch.zeros((n_pos, H), dtype=torch.bfloat16, device="cuda")
+    flags = torch.empty((n_pos // 128,), dtype=torch.int32, device="cuda")
+    L.call("b200moe_scatter_rows_bf16", L.ptr(x), T, H, L.ptr(table), K, n_pos, L.ptr(b2e), B, E,
+           L.ptr(aff) if scaled else None, L.F32, L.ptr(out), L.ptr(flags), L.stream_ptr())
+    ref = torch.zeros_like(out)
+    want = torch.zeros_like(flags)
+    for t in range(T):
+        for p in table[t].tolist():
+            if 0 <= p < n_pos:
+                a = aff[t, int(b2e[p // B])].to(torch.bfloat16).float() if scaled else 1.0
+                ref[p] = (x[t].float() * a).to(torch.bfloat16)
+                want[p >> 7] = max(int(want[p >> 7]), (p & 127) + 1)
+    assert torch.equal(out, ref) and torch.equal(flags, want)
+
+
+@pytest.mark.parametrize("T,H,offset", [(1, 8, 0), (5, 250, 0), (3, 1001, 0), (4, 4096, 0), (2, 9000, 0), (3, 512, 1)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_odd_rows(T, H, offset, residual):
+    """Row lengths that are no multiple of a vector or of the CTA, and rows that start off a 16-byte boundary."""
+    L = _lib()
+    x = torch.randn((T * H + offset,), device="cuda", generator=_gen(5)).to(torch.bfloat16)[offset:].view(T, H)
+    r = torch.randn((T, H), device="cuda", generator=_gen(6)).to(torch.bfloat16) if residual else None
+    gamma = torch.rand((H,), device="cuda", generator=_gen(7)) + 0.5
+    out, res = torch.empty((T, H), dtype=torch.bfloat16, device="cuda"), torch.empty((T, H), dtype=torch.bfloat16, device="cuda")
+    L.call("b200moe_rmsnorm", L.ptr(x), L.ptr(r), L.ptr(gamma), L.F32, T, H, 0, 1e-6, L.ptr(out),
+           L.ptr(res) if residual else None, L.stream_ptr())
+    v = (x.float() + r.float()).to(torch.bfloat16) if residual else x
+    if residual:
+        assert torch.equal(res, v)
+    ref = v.double() / torch.sqrt(v.double().pow(2).mean(1, keepdim=True) + 1e-6) * gamma.double()
+    assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-30).all())
