@@ -101,3 +101,19 @@ def test_rmsnorm_odd_rows(T, H, offset, residual):
         assert torch.equal(res, v)
     ref = v.double() / torch.sqrt(v.double().pow(2).mean(1, keepdim=True) + 1e-6) * gamma.double()
     assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-30).all())
+
+
+@pytest.mark.parametrize("T,n_cand,H", [(1, 1, 8), (3, 7, 1032), (2, 9, 3072), (5, 130, 2056), (1200, 17, 256)])
+def test_combine_lists(T, n_cand, H):
+    L = _lib()
+    rows = T * n_cand
+    y = torch.randn((rows, H), device="cuda", generator=_gen(8)).to(torch.bfloat16)
+    table = _positions(T, n_cand, rows, 0.7, T)
+    table = torch.where(table >= rows, -1, table)
+    out = torch.empty((T, H), dtype=torch.bfloat16, device="cuda")
+    L.call("b200moe_combine", L.ptr(y), L.ptr(table), T, n_cand, H, L.ptr(out), L.stream_ptr())
+    ref = torch.zeros((T, H), dtype=torch.float32, device="cuda")
+    for c in range(n_cand):
+        p = table[:, c]
+        ref = ref + torch.where((p >= 0)[:, None], y[p.clamp(min=0).long()].float(), 0.0)
+    assert torch.equal(out, ref.to(torch.bfloat16))
