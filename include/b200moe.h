@@ -162,6 +162,16 @@ int b200moe_group_tokens_static(const void* routing, int routing_mode, int routi
 int b200moe_build_position_table(const int32_t* token_position_to_id, const int32_t* block_to_expert,
                                  const int32_t* conditions, int n_blocks, int B, int T, int E, int32_t* pos_table,
                                  b200moe_stream_t stream);
+/* Bookkeeping of the all-expert decode mode (core/moe/moe_tkg/moe_tkg_affinity_masking.py:31-117) in one launch.
+ * Layout (NULL = leave out): every local expert owns ceil(T / B) blocks that hold tokens 0..T-1 in order --
+ * token_position_to_id [E_local * T_pad], block_to_expert [E_local * T_pad / B], pos_table [T, E_local].
+ * local_affinities [T, E_local] fp32 (NULL = leave out): columns [E_local * r, E_local * (r + 1)) of the [T, E] table,
+ * r = *rank_id (device integer of rank_bytes bytes; NULL = 0), multiplied by 0 where expert_index [T, K] (NULL = keep
+ * all) does not name the expert; columns outside the table come back as NaN. */
+int b200moe_all_expert_setup(int T, int E_local, int B, int32_t* token_position_to_id, int32_t* block_to_expert,
+                             int32_t* pos_table, const void* affinities, int aff_dtype, int E, const void* rank_id,
+                             int rank_bytes, const int32_t* expert_index, int K, float* local_affinities,
+                             b200moe_stream_t stream);
 
 /* ---- MXFP8 activation quantisation --------------------------------------------
  * load_and_quantize_hidden_states (core/moe/moe_cte/moe_cte_mx_utils.py:456-945) with

@@ -51,7 +51,7 @@ def moe_group_tokens(routing: torch.Tensor, num_experts: int, block_size: int, n
     cond = torch.empty(N + 2 if mx_conditions else N + 1, dtype=torch.int32, device=dev)
     counts = torch.empty(E, dtype=torch.int32, device=dev)
     inv = torch.empty((T, K), dtype=torch.int32, device=dev) if (index_mode and want_inverse) else None
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    status = torch.empty(1, dtype=torch.int32, device=dev)  # always written
     ws = torch.empty(lib.b200moe_group_tokens_workspace_bytes(T, E), dtype=torch.uint8, device=dev)
     _lib.call("b200moe_group_tokens", _lib.ptr(routing), _lib.ROUTING_INDEX if index_mode else _lib.ROUTING_MASK,
               _lib.I32 if index_mode else _lib.dtype_code(routing), T, E, K if index_mode else 0, B, N,

@@ -130,17 +130,9 @@ def moe_tkg(
             A(rank_id is not None, f"{_PREFIX} rank_id is required for all-expert mode with affinity scaling")
         # local expert columns [E_L * rank_id, E_L * (rank_id + 1)), taken with a device-side index so that the
         # rank tensor never has to travel to the host (moe_tkg_affinity_masking.py:31-117)
-        aff = None
-        if post_scale or is_all_expert_dynamic:
-            cols = torch.arange(E_L, dtype=torch.int64, device=dev)
-            if rank_id is not None:
-                cols = cols + rank_id.reshape(-1)[:1].to(torch.int64) * E_L
-            aff = expert_affinities.float().index_select(1, cols)
-            if mask_unselected_experts:
-                sel = torch.zeros((T, E), dtype=torch.float32, device=dev)
-                sel.scatter_(1, expert_index.to(torch.int64), 1.0)
-                aff = aff * sel.index_select(1, cols)
-            aff = aff.contiguous()
+        want_aff = post_scale or is_all_expert_dynamic
+        aff = local_affinities(expert_affinities, E_L, T, rank_id,
+                               expert_index if mask_unselected_experts else None) if want_aff else None
         if is_all_expert_dynamic:
             # dynamic control flow: per expert only the tokens routed to it (non-zero masked affinity) are
             # gathered into blocks and computed (all_expert_mx_impl.py:276-350); the block bookkeeping is the
@@ -153,12 +145,15 @@ def moe_tkg(
             _lib.call("b200moe_build_position_table", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(cond), n_blocks, _BLOCK,
                       T, E_L, _lib.ptr(table), _lib.stream_ptr())
         else:
-            tpi, b2e, table = all_expert_layout(T, E_L, dev)
             cond = None
         kw = {}
-        if _prequantized is not None and not is_all_expert_dynamic and not dense:
-            # the caller (moe_block_tkg) has run the fused RMSNorm + quantise kernel into this workspace
-            kw = dict(workspace=_prequantized, prequantized=True)
+        if not is_all_expert_dynamic:
+            if _prequantized is not None and not dense:
+                # the caller (moe_block_tkg) has run the fused RMSNorm + quantise kernel into this workspace
+                ws, (tpi, b2e, table) = _prequantized
+                kw = dict(workspace=ws, prequantized=True)
+            else:
+                tpi, b2e, table = all_expert_layout(T, E_L, dev)
         _run(weights, hidden, T, weights, tpi, b2e, cond, _BLOCK, aff if post_scale else None, table, out,
              activation_fn.value, clamps[0], clamps[1], _impl, _check_status, **kw)
     if output_dtype is not None and output_dtype != torch.bfloat16:
@@ -169,15 +164,40 @@ def moe_tkg(
 def all_expert_layout(T: int, E_L: int, device):
     """Static block layout of the all-expert mode: every local expert owns ceil(T / 128) blocks that hold tokens
     0..T-1 in order.  Returns ``(token_position_to_id, block_to_expert, table [T, E_L])``."""
-    n_sub = math.ceil(T / _BLOCK)
-    Tpad = n_sub * _BLOCK
-    ids = torch.full((Tpad,), -1, dtype=torch.int32, device=device)
-    ids[:T] = torch.arange(T, dtype=torch.int32, device=device)
-    tpi = ids.repeat(E_L)
-    b2e = torch.arange(E_L, dtype=torch.int32, device=device).repeat_interleave(n_sub)
-    table = (torch.arange(E_L, dtype=torch.int32, device=device)[None, :] * Tpad +
-             torch.arange(T, dtype=torch.int32, device=device)[:, None]).contiguous()
+    Tpad = math.ceil(T / _BLOCK) * _BLOCK
+    tpi = torch.empty(E_L * Tpad, dtype=torch.int32, device=device)
+    b2e = torch.empty(E_L * Tpad // _BLOCK, dtype=torch.int32, device=device)
+    table = torch.empty((T, E_L), dtype=torch.int32, device=device)
+    _lib.call("b200moe_all_expert_setup", T, E_L, _BLOCK, _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(table), None, _lib.F32, 0,
+              None, 0, None, 0, None, _lib.stream_ptr())
     return tpi, b2e, table
+
+
+def local_affinities(expert_affinities: torch.Tensor, E_L: int, T: int, rank_id, expert_index) -> torch.Tensor:
+    """fp32 ``[T, E_L]``: this rank's columns of the affinity table, multiplied by 0 where ``expert_index`` (None = keep
+    all) does not name the expert.  The rank is read on the device and never travels to the host."""
+    E = expert_affinities.shape[1]
+    aff = expert_affinities.expand(T, E) if expert_affinities.shape[0] == 1 else expert_affinities
+    _lib.kernel_assert(aff.shape[0] == T or (expert_index is None and aff.shape[0] > T),
+                       f"{_PREFIX} expert_affinities must hold one row per token")
+    aff = aff.contiguous()
+    if aff.dtype not in (torch.float32, torch.bfloat16):
+        aff = aff.float()
+    rank = None if rank_id is None else rank_id.reshape(-1)[:1]
+    if rank is not None and rank.dtype not in (torch.int32, torch.int64):
+        rank = rank.to(torch.int64)
+    idx, K = None, 0
+    if expert_index is not None:
+        idx = expert_index if expert_index.dtype in (torch.int32, torch.uint32) else expert_index.to(torch.int32)
+        _lib.kernel_assert(idx.shape[0] <= T, f"{_PREFIX} expert_index must hold one row per token")
+        if idx.shape[0] < T:  # a token without a row selects nothing
+            idx = torch.nn.functional.pad(idx.view(torch.int32), (0, 0, 0, T - idx.shape[0]), value=-1)
+        idx, K = idx.contiguous(), idx.shape[1]
+    out = torch.empty((T, E_L), dtype=torch.float32, device=aff.device)
+    _lib.call("b200moe_all_expert_setup", T, E_L, _BLOCK, None, None, None, _lib.ptr(aff), _lib.dtype_code(aff), E,
+              _lib.ptr(rank), 0 if rank is None else rank.element_size(), _lib.ptr(idx), K, _lib.ptr(out),
+              _lib.stream_ptr())
+    return out
 
 
 def _run(weights, *args, **kw):

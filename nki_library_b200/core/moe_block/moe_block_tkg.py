@@ -98,13 +98,14 @@ def moe_block_tkg(
                 expert_gate_up_weights, expert_gate_up_weights_scale, expert_down_weights, expert_down_weights_scale,
                 expert_gate_up_bias, expert_down_bias)
         w = expert_gate_up_weights
-        _, _, table = all_expert_layout(T, w.E, x.device)
+        layout = all_expert_layout(T, w.E, x.device)
+        table = layout[2]
         n_pos = w.E * math.ceil(T / 128) * 128
-        prequantized = pipeline.get_workspace(n_pos, H, w.I, x.device)
+        ws = pipeline.get_workspace(n_pos, H, w.I, x.device)
+        prequantized = (ws, layout)
         _lib.call("b200moe_rmsnorm_quantize_mxfp8", _lib.ptr(x), _lib.ptr(res), _lib.ptr(g), g_code, T, H, h_act,
                   float(eps), _lib.ptr(normed), _lib.ptr(residual_out), _lib.ptr(table), table.shape[1], n_pos,
-                  int(w.h_packed_order), _lib.ptr(prequantized.xq), _lib.ptr(prequantized.x_sf),
-                  _lib.ptr(prequantized.tile_flags), _lib.stream_ptr())
+                  int(w.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
     else:
         _lib.call("b200moe_rmsnorm", _lib.ptr(x), _lib.ptr(res), _lib.ptr(g), g_code, T, H, h_act, float(eps),
                   _lib.ptr(normed), _lib.ptr(residual_out), _lib.stream_ptr())

@@ -117,3 +117,54 @@ def test_combine_lists(T, n_cand, H):
         p = table[:, c]
         ref = ref + torch.where((p >= 0)[:, None], y[p.clamp(min=0).long()].float(), 0.0)
     assert torch.equal(out, ref.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T,E,K,B", [(1, 1, 1, 128), (256, 33, 3, 128), (257, 4, 2, 128), (2305, 17, 5, 256),
+                                     (4500, 513, 8, 128), (9000, 128, 8, 128), (700, 1000, 4, 128)])
+def test_group_tokens_scan(T, E, K, B):
+    """Chunks of 256 tokens are scanned by several threads per column when the columns leave room for that."""
+    import nki_library_b200 as m
+    idx = torch.rand((T, E), device="cuda", generator=_gen(T)).topk(K, dim=1).indices.to(torch.int32)
+    N = m.get_n_blocks(T, K, E, B)
+    g = m.moe_group_tokens(idx, E, B, N, top_k=K, check=True)
+    tpi, b2e, pos, counts = [], [], torch.full((T, E), -1, dtype=torch.int64), []
+    sel = torch.zeros((T, E), dtype=torch.bool)
+    sel.scatter_(1, idx.cpu().long(), True)
+    for e in range(E):
+        ids = sel[:, e].nonzero().flatten()
+        blocks = (len(ids) + B - 1) // B
+        pos[ids, e] = len(tpi) + torch.arange(len(ids))
+        tpi += ids.tolist() + [-1] * (blocks * B - len(ids))
+        b2e += [e] * blocks
+        counts.append(len(ids))
+    used = len(b2e)
+    tpi += [-1] * ((N - used) * B)
+    b2e += [E - 1] * (N - used)
+    assert g["token_position_to_id"].tolist() == tpi and g["block_to_expert"].tolist() == b2e
+    assert g["counts"].tolist() == counts and g["conditions"].tolist() == [1] * used + [0] * (N - used + 2)
+    assert torch.equal(g["inverse_map"].cpu().long(), pos.gather(1, idx.cpu().long()))
+    # too few blocks are reported
+    if used > 1:
+        assert int(m.moe_group_tokens(idx, E, B, used - 1, top_k=K)["status"]) == 1
+
+
+@pytest.mark.parametrize("T,E_L,E,rank_dtype", [(1, 1, 1, torch.int32), (129, 16, 128, torch.int32), (37, 3, 10, torch.int64),
+                                                (128, 128, 128, torch.uint8)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_all_expert_setup(T, E_L, E, rank_dtype, masked):
+    mod = importlib.import_module("nki_library_b200.core.moe.moe_tkg.moe_tkg")
+    r = E // E_L - 1
+    K = min(4, E)
+    aff = torch.rand((T, E), device="cuda", generator=_gen(11)).to(torch.bfloat16 if E == 10 else torch.float32)
+    idx = torch.rand((T, E), device="cuda", generator=_gen(12)).topk(K, dim=1).indices
+    rank = torch.tensor([[r]], dtype=rank_dtype, device="cuda")
+    got = mod.local_affinities(aff, E_L, T, rank, idx.to(torch.int32) if masked else None)
+    sel = torch.zeros((T, E), device="cuda").scatter_(1, idx, 1.0) if masked else 1.0
+    assert torch.equal(got, (aff.float() * sel)[:, r * E_L:(r + 1) * E_L])
+    tpi, b2e, table = mod.all_expert_layout(T, E_L, aff.device)
+    pad = (T + 127) // 128 * 128
+    ids = torch.full((pad,), -1, dtype=torch.int32, device="cuda")
+    ids[:T] = torch.arange(T, device="cuda")
+    assert torch.equal(tpi, ids.repeat(E_L))
+    assert b2e.tolist() == [e for e in range(E_L) for _ in range(pad // 128)]
+    assert torch.equal(table, (torch.arange(E_L, device="cuda")[None] * pad + torch.arange(T, device="cuda")[:, None]).int())
