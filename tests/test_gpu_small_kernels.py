@@ -168,3 +168,23 @@ def test_all_expert_setup(T, E_L, E, rank_dtype, masked):
     assert torch.equal(tpi, ids.repeat(E_L))
     assert b2e.tolist() == [e for e in range(E_L) for _ in range(pad // 128)]
     assert torch.equal(table, (torch.arange(E_L, device="cuda")[None] * pad + torch.arange(T, device="cuda")[:, None]).int())
+
+
+@pytest.mark.parametrize("E", [1, 3, 4, 12, 65, 250, 511])
+def test_router_narrow_and_odd_widths(E):
+    """Router weight rows that are no whole number of 16-byte pieces; ids exact, logits within the fp32 sum's error."""
+    import nki_library_b200 as m
+    T, H = 37, 640
+    x = torch.randn((T, H), device="cuda", generator=_gen(9)).to(torch.bfloat16)
+    w = (torch.randn((H, E), device="cuda", generator=_gen(10)) * 0.1).to(torch.bfloat16)
+    k = min(E, 4)
+    logits, aff = torch.empty((T, E), device="cuda"), torch.empty((T, E), device="cuda")
+    idx = torch.empty((T, k), dtype=torch.int32, device="cuda")
+    m.router_topk(x, w, None, logits, aff, idx, m.RouterActFnType.SOFTMAX, k, 1, 0, norm_topk_prob=True)
+    ref = x.double() @ w.double()
+    # H products added in fp32: at most H * 2^-24 of the sum of magnitudes
+    assert bool(((logits.double() - ref).abs() <= H * 2.0 ** -24 * (x.double().abs() @ w.double().abs())).all())
+    assert torch.equal(idx.long(), logits.topk(k, dim=1).indices)
+    p = torch.softmax(logits, 1).gather(1, idx.long())
+    want = torch.zeros_like(aff).scatter_(1, idx.long(), p / p.sum(1, keepdim=True))
+    assert bool(((aff - want).abs() <= 1e-5 * want + 1e-12).all())
