@@ -439,6 +439,8 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
   }
   const int cta_rank = CTAS == 2 ? static_cast<int>(cluster_cta_rank()) : 0;
   const int unit = blockIdx.x / CTAS, n_units = gridDim.x / CTAS;
+  // cleared here and not by a memset node in front of every launch: a wait that reports expires after seconds
+  if (blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&full[s], 1);
@@ -1168,8 +1170,8 @@ int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, 
   p.k_blocks = (Kb + kBlockK - 1) / kBlockK;
   p.w_row_atoms = (p.n_total + 127) / 128;
   p.w_sf_expert_stride = static_cast<int64_t>(p.w_row_atoms) * p.k_blocks * 512;
-  B200MOE_CUDA_OK(cudaMemsetAsync(p.status, 0, 4, st));
   if (impl & B200MOE_IMPL_SIMT) {
+    B200MOE_CUDA_OK(cudaMemsetAsync(p.status, 0, 4, st));
     const int64_t work = epi == 0 ? static_cast<int64_t>(p.m_tiles_total) * 128 * (p.I / 32)
                                   : static_cast<int64_t>(p.m_tiles_total) * 128 * p.H_out;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 32;
@@ -1198,11 +1200,18 @@ int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, 
   CUtensorMap* const w_maps[4] = {&wm.rows128, &wm.rows64, &wm.rows32, &wm.rows16};
   CUtensorMap* const x_maps[4] = {&xm.rows128, &xm.rows64, &xm.rows32, &xm.rows16};
   CUtensorMap sfx, sfw;
+  // weight boxes: a pair copies 128 rows at a time, a single CTA's gate/up tiles have 128 or 64, its down tiles any
+  // multiple of 16
+  const int n_w_maps = pair ? 1 : (epi == 0 ? 2 : 4);
   for (int i = 0; i < 4; ++i) {
     int rc = make_rows_map(x_maps[i], x, Kb, static_cast<int64_t>(p.m_tiles_total) * 128, 0, 128 >> i);
     if (rc != B200MOE_OK) return rc;
-    rc = make_rows_map(w_maps[i], w, Kb, p.n_total, p.E, 128 >> i, nibbles);
-    if (rc != B200MOE_OK) return rc;
+    if (i < n_w_maps) {
+      rc = make_rows_map(w_maps[i], w, Kb, p.n_total, p.E, 128 >> i, nibbles);
+      if (rc != B200MOE_OK) return rc;
+    } else {
+      *w_maps[i] = wm.rows128;  // never used
+    }
   }
   if (kind == 0) {
     int rc = make_atoms_map(&sfx, p.x_sf, static_cast<int64_t>(p.m_tiles_total) * p.k_blocks);
