@@ -105,6 +105,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_functions: dict = {}  # entry points by name, bound once
 
 
 def load_library() -> ctypes.CDLL:
@@ -125,14 +126,13 @@ def load_library() -> ctypes.CDLL:
 
 
 def ptr(t):
-    """Device pointer of a tensor (None -> NULL)."""
-    if t is None:
-        return None
-    return c_void_p(t.data_ptr())
+    """Device pointer of a tensor as a plain integer, which ctypes converts without an object in between
+    (None -> NULL)."""
+    return None if t is None else t.data_ptr()
 
 
 def stream_ptr():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch.cuda.current_stream().cuda_stream
 
 
 def dtype_code(t: torch.Tensor) -> int:
@@ -152,10 +152,12 @@ def kernel_assert(cond: bool, msg: str) -> None:
 
 def call(name: str, *args) -> None:
     """Invoke an ``int``-returning entry point and raise on a non-zero status."""
-    lib = load_library()
-    rc = getattr(lib, name)(*args)
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(load_library(), name)
+    rc = fn(*args)
     if rc != 0:
-        msg = lib.b200moe_last_error().decode("utf-8", "replace")
+        msg = load_library().b200moe_last_error().decode("utf-8", "replace")
         raise AssertionError(ERROR_PREFIX + f"{name} failed ({rc}): {msg}")
 
 

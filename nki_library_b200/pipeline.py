@@ -96,13 +96,13 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
               _lib.ptr(weights.w1_sf), weights.w_format, _lib.ptr(weights.bias_gu), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), n_blocks, block_size, E, H, I, act_fn, _clamp(gate_clamp[0]),
               _clamp(gate_clamp[1]), _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.mq), _lib.ptr(ws.m_sf),
-              _lib.ptr(ws.status[1:]), impl, None, st)
+              _lib.ptr(ws.status) + 4, impl, None, st)
     mark("t2")
     _lib.call("b200moe_grouped_gemm2_scale", _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(weights.w2),
               _lib.ptr(weights.w2_sf), weights.w_format, _lib.ptr(weights.bias_d), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), _lib.ptr(token_position_to_id), hidden_rows, n_blocks, block_size, E, H, I,
               _lib.ptr(affinities), _lib.F32 if affinities is None else _lib.dtype_code(affinities),
-              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status[2:]), impl, None, st)
+              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8, impl, None, st)
     mark("t3")
     _lib.call("b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(table), out.shape[0], table.shape[1], H, _lib.ptr(out), st)
     if check_status:
@@ -154,11 +154,11 @@ def run_blocks_dense(hidden: torch.Tensor, hidden_rows: int, weights, token_posi
     _lib.call("b200moe_dense_gemm1_swiglu", _lib.ptr(ws.x_pos), _lib.ptr(weights.w1), _lib.ptr(weights.scale_gu),
               _lib.ptr(weights.bias_gu), _lib.ptr(block_to_expert), _lib.ptr(conditions), _lib.ptr(ws.tile_flags),
               n_blocks, block_size, E, H, I, act_fn, _clamp(gate_clamp[0]), _clamp(gate_clamp[1]),
-              _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.m), _lib.ptr(ws.status[1:]), impl, st)
+              _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.m), _lib.ptr(ws.status) + 4, impl, st)
     _lib.call("b200moe_dense_gemm2_scale", _lib.ptr(ws.m), _lib.ptr(weights.w2), _lib.ptr(weights.scale_d),
               _lib.ptr(weights.bias_d), _lib.ptr(block_to_expert), _lib.ptr(conditions), _lib.ptr(ws.tile_flags),
               _lib.ptr(token_position_to_id), hidden_rows, n_blocks, block_size, E, H, I,
-              None if pre_scale else _lib.ptr(affinities), aff_code, 0, _lib.ptr(ws.y_pos), _lib.ptr(ws.status[2:]),
+              None if pre_scale else _lib.ptr(affinities), aff_code, 0, _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8,
               impl, st)
     _lib.call("b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(table), out.shape[0], table.shape[1], H, _lib.ptr(out), st)
     if check_status:
