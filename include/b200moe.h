@@ -60,14 +60,19 @@ enum { B200MOE_W_E4M3 = 0, B200MOE_W_E5M2 = 1, B200MOE_W_E2M1 = 5 };
  *   B200MOE_GEMM_NO_PAIR     never run on CTA pairs (tcgen05 cta_group::2, 256 weight rows x up to 256 tokens)
  *   B200MOE_GEMM_FORCE_PAIR  CTA pairs whatever the shape (default: when the block size is a multiple of 256, or
  *                            the block list holds two or more 128-position tiles per expert)
- *   B200MOE_GEMM_NO_SPLIT, B200MOE_GEMM_NO_OVERLAP  accepted and ignored: there is one launch per contraction */
+ *   B200MOE_GEMM_NO_SPLIT, B200MOE_GEMM_NO_OVERLAP  accepted and ignored: there is one launch per contraction
+ *   B200MOE_GEMM_CHAINED     the launch may overlap the end of the kernel launched directly in front on this stream:
+ *                            everything it reads but x (and, down, m) with their scales was complete before that kernel
+ *                            was launched.  Only the quantisers, b200moe_all_expert_setup and the gate/up contractions
+ *                            let a chained launch in early */
 enum {
   B200MOE_IMPL_SIMT = 1,
   B200MOE_GEMM_TILE_N128 = 0x100,
   B200MOE_GEMM_NO_PAIR = 0x200,
   B200MOE_GEMM_FORCE_PAIR = 0x400,
   B200MOE_GEMM_NO_SPLIT = 0x800,
-  B200MOE_GEMM_NO_OVERLAP = 0x1000
+  B200MOE_GEMM_NO_OVERLAP = 0x1000,
+  B200MOE_GEMM_CHAINED = 0x2000
 };
 /* routing source accepted by b200moe_group_tokens */
 enum { B200MOE_ROUTING_INDEX = 0, B200MOE_ROUTING_MASK = 1 };
@@ -132,6 +137,13 @@ int b200moe_group_tokens(const void* routing, int routing_mode, int routing_dtyp
                          int skip_token, int mx_conditions, int32_t* token_position_to_id, int32_t* block_to_expert,
                          int32_t* conditions, int32_t* counts, int32_t* inverse_map, int32_t* status, void* workspace,
                          size_t workspace_bytes, b200moe_stream_t stream);
+/* The same, and tile_flags [N * B / 128] (NULL = leave out; B % 128 == 0): the occupied leading rows of every 128
+ * positions. */
+int b200moe_group_tokens_tiles(const void* routing, int routing_mode, int routing_dtype, int T, int E, int K, int B, int N,
+                               int skip_token, int mx_conditions, int32_t* token_position_to_id,
+                               int32_t* block_to_expert, int32_t* conditions, int32_t* counts, int32_t* inverse_map,
+                               int32_t* tile_flags, int32_t* status, void* workspace, size_t workspace_bytes,
+                               b200moe_stream_t stream);
 
 /* Same grouping for callers that must not allocate device memory -- code running
  * inside a memory-pool or allocator callback, a plug-in whose host forbids
@@ -162,6 +174,11 @@ int b200moe_group_tokens_static(const void* routing, int routing_mode, int routi
 int b200moe_build_position_table(const int32_t* token_position_to_id, const int32_t* block_to_expert,
                                  const int32_t* conditions, int n_blocks, int B, int T, int E, int32_t* pos_table,
                                  b200moe_stream_t stream);
+/* The same, and tile_flags [n_blocks * B / 128] (NULL = leave out; B % 128 == 0): per 128 positions the leading rows up
+ * to the last one that holds a token, as the quantisers would write them. */
+int b200moe_build_position_table_tiles(const int32_t* token_position_to_id, const int32_t* block_to_expert,
+                                       const int32_t* conditions, int n_blocks, int B, int T, int E,
+                                       int32_t* pos_table, int32_t* tile_flags, b200moe_stream_t stream);
 /* Bookkeeping of the all-expert decode mode (core/moe/moe_tkg/moe_tkg_affinity_masking.py:31-117) in one launch.
  * Layout (NULL = leave out): every local expert owns ceil(T / B) blocks that hold tokens 0..T-1 in order --
  * token_position_to_id [E_local * T_pad], block_to_expert [E_local * T_pad / B], pos_table [T, E_local].

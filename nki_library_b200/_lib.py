@@ -26,6 +26,7 @@ W_E4M3, W_E5M2, W_E2M1 = 0, 1, 5  # weight element formats (B200MOE_W_*)
 ROUTING_INDEX, ROUTING_MASK = 0, 1
 # per-call variant word of the grouped contractions (B200MOE_IMPL_* / B200MOE_GEMM_*)
 IMPL_SIMT, GEMM_TILE_N128, GEMM_NO_PAIR, GEMM_FORCE_PAIR, GEMM_NO_SPLIT, GEMM_NO_OVERLAP = 1, 0x100, 0x200, 0x400, 0x800, 0x1000
+GEMM_CHAINED = 0x2000  # may overlap the kernel in front; see the header for what that asks of the caller
 ROUTER_AUTO, ROUTER_SPLIT_K, ROUTER_TCGEN05 = 0, 1, 2
 
 # name -> (restype, argtypes); must list every symbol of include/b200moe.h
@@ -47,11 +48,16 @@ SIGNATURES = {
     "b200moe_group_tokens": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                      c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
                                      c_void_p]),
+    "b200moe_group_tokens_tiles": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                           c_void_p, c_size_t, c_void_p]),
     "b200moe_group_tokens_static_max_bytes": (c_size_t, []),
     "b200moe_group_tokens_static": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                             c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "b200moe_build_position_table": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                              c_void_p]),
+    "b200moe_build_position_table_tiles": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
+                                                   c_void_p, c_void_p]),
     "b200moe_all_expert_setup": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                          c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "b200moe_gather_quantize_mxfp8": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int64, c_int, c_void_p, c_void_p,

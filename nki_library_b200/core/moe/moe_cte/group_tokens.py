@@ -12,7 +12,7 @@ from .moe_cte_utils import get_n_blocks
 
 def moe_group_tokens(routing: torch.Tensor, num_experts: int, block_size: int, n_blocks: Optional[int] = None,
                      top_k: Optional[int] = None, skip_token: bool = True, mx_conditions: bool = True,
-                     want_inverse: bool = True, check: bool = False):
+                     want_inverse: bool = True, check: bool = False, _tile_flags: Optional[torch.Tensor] = None):
     """Block assignment for the blockwise expert kernels.
 
     ``routing`` is either ``expert_index [T, K]`` (int32/uint32) or a ``[T, E]``
@@ -53,10 +53,10 @@ def moe_group_tokens(routing: torch.Tensor, num_experts: int, block_size: int, n
     inv = torch.empty((T, K), dtype=torch.int32, device=dev) if (index_mode and want_inverse) else None
     status = torch.empty(1, dtype=torch.int32, device=dev)  # always written
     ws = torch.empty(lib.b200moe_group_tokens_workspace_bytes(T, E), dtype=torch.uint8, device=dev)
-    _lib.call("b200moe_group_tokens", _lib.ptr(routing), _lib.ROUTING_INDEX if index_mode else _lib.ROUTING_MASK,
+    _lib.call("b200moe_group_tokens_tiles", _lib.ptr(routing), _lib.ROUTING_INDEX if index_mode else _lib.ROUTING_MASK,
               _lib.I32 if index_mode else _lib.dtype_code(routing), T, E, K if index_mode else 0, B, N,
               int(skip_token), int(mx_conditions), _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(cond), _lib.ptr(counts),
-              _lib.ptr(inv), _lib.ptr(status), _lib.ptr(ws), ws.numel(), _lib.stream_ptr())
+              _lib.ptr(inv), _lib.ptr(_tile_flags), _lib.ptr(status), _lib.ptr(ws), ws.numel(), _lib.stream_ptr())
     if check:
         _lib.kernel_assert(int(status.item()) == 0, f"n_blocks ({N}) is too small for this routing")
     return {"token_position_to_id": tpi, "block_to_expert": b2e, "conditions": cond, "counts": counts,

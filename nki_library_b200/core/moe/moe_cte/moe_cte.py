@@ -160,13 +160,14 @@ def moe_cte(
     hidden = hidden_states.contiguous()
     out = torch.empty((rows, H), dtype=torch.bfloat16, device=hidden.device)
     table = torch.empty((rows, E), dtype=torch.int32, device=hidden.device)
-    _lib.call("b200moe_build_position_table", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
-              hidden_rows, E, _lib.ptr(table), _lib.stream_ptr())
+    ws = pipeline.get_workspace(N * block_size, H, weights.I, hidden.device)
+    _lib.call("b200moe_build_position_table_tiles", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
+              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
     if rows != hidden_rows:
         table[hidden_rows:].fill_(-1)
     pipeline.run_blocks(hidden, hidden_rows, weights, tpi, b2e, conditions, block_size, aff, table, out,
                         activation_function.value, (gate_clamp_lower_limit, gate_clamp_upper_limit),
-                        (up_clamp_lower_limit, up_clamp_upper_limit), _impl, _check_status)
+                        (up_clamp_lower_limit, up_clamp_upper_limit), _impl, _check_status, ws, flags_ready=True)
     if compat_lnc_slabs:
         return torch.stack([out, torch.zeros_like(out)])
     return out
@@ -205,12 +206,14 @@ def _moe_cte_dense(hidden_states, expert_affinities_masked, gate_up_proj_weight,
     hidden = hidden_states.to(torch.bfloat16).contiguous()
     out = torch.empty((rows, H), dtype=torch.bfloat16, device=hidden.device)
     table = torch.empty((rows, E), dtype=torch.int32, device=hidden.device)
-    _lib.call("b200moe_build_position_table", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
-              hidden_rows, E, _lib.ptr(table), _lib.stream_ptr())
+    ws = pipeline.get_dense_workspace(N * block_size, H, weights.I, hidden.device)
+    _lib.call("b200moe_build_position_table_tiles", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
+              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
     if rows != hidden_rows:
         table[hidden_rows:].fill_(-1)
     pipeline.run_blocks_dense(hidden, hidden_rows, weights, tpi, b2e, conditions, block_size, aff, table, out,
-                              activation_function.value, gate_clamp, up_clamp, impl, check_status, pre_scale)
+                              activation_function.value, gate_clamp, up_clamp, impl, check_status, pre_scale, ws,
+                              flags_ready=True)
     if compat_lnc_slabs:
         return torch.stack([out, torch.zeros_like(out)])
     return out

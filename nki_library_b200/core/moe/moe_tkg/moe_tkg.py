@@ -116,14 +116,17 @@ def moe_tkg(
         K = idx.shape[1]
         E = expert_affinities.shape[1]
         A(E == E_L, f"{_PREFIX} selective mode needs all {E} experts local, got {E_L}")
-        g = moe_group_tokens(idx, E, _BLOCK, get_n_blocks(T, K, E, _BLOCK), skip_token=True)
+        n_blocks = get_n_blocks(T, K, E, _BLOCK)
+        ws = (pipeline.get_dense_workspace if dense else pipeline.get_workspace)(n_blocks * _BLOCK, H, weights.I, dev)
+        g = moe_group_tokens(idx, E, _BLOCK, n_blocks, skip_token=True, _tile_flags=ws.tile_flags)
         aff = None
         if post_scale:
             aff = expert_affinities.contiguous()
             if aff.dtype not in (torch.float32, torch.bfloat16):
                 aff = aff.float()
         _run(weights, hidden, T, weights, g["token_position_to_id"], g["block_to_expert"], g["conditions"],
-             _BLOCK, aff, g["inverse_map"], out, activation_fn.value, clamps[0], clamps[1], _impl, _check_status)
+             _BLOCK, aff, g["inverse_map"], out, activation_fn.value, clamps[0], clamps[1], _impl, _check_status,
+             workspace=ws, flags_ready=True)
     else:
         E = expert_affinities.shape[1]
         if post_scale:
@@ -151,7 +154,7 @@ def moe_tkg(
             if _prequantized is not None and not dense:
                 # the caller (moe_block_tkg) has run the fused RMSNorm + quantise kernel into this workspace
                 ws, (tpi, b2e, table) = _prequantized
-                kw = dict(workspace=ws, prequantized=True)
+                kw = dict(workspace=ws, prequantized=True, flags_ready=True)
             else:
                 tpi, b2e, table = all_expert_layout(T, E_L, dev)
         _run(weights, hidden, T, weights, tpi, b2e, cond, _BLOCK, aff if post_scale else None, table, out,

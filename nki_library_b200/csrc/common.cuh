@@ -86,6 +86,11 @@ __host__ __device__ inline int64_t sf_atom_offset(int64_t row, int64_t kb32, int
   return atom * 512 + (r & 31) * 16 + (r >> 5) * 4 + (kb32 & 3);
 }
 
+// Programmatic dependent launch: the grids behind this one may start once every CTA has said so or exited ...
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// ... and this returns once the grid in front is complete and its writes are visible.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float load_as_float(const void* p, int64_t i, int dtype) {
   if (dtype == B200MOE_F32) return static_cast<const float*>(p)[i];
   if (dtype == B200MOE_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);

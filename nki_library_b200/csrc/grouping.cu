@@ -109,7 +109,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* s_warp, int& tot
 // mode 0: find_nonzero_indices (column c writes at c*T); mode 1: block grouping.
 __device__ __forceinline__ int64_t plan_columns(int total, int n_cols, int mode, int T, int B, int N, int mx_conditions,
                                                 int32_t* counts, int32_t* block_to_expert, int32_t* conditions,
-                                                int32_t* status) {
+                                                int32_t* tile_flags, int32_t* status) {
   __shared__ int s_warp[32];
   const int c = threadIdx.x;
   if (counts && c < n_cols) counts[c] = total;
@@ -123,6 +123,11 @@ __device__ __forceinline__ int64_t plan_columns(int total, int n_cols, int mode,
     const int nb = blocks + (c == n_cols - 1 ? n_pad : 0);
     for (int b = 0; b < nb; ++b)
       if (first + b < N) block_to_expert[first + b] = c;
+    if (tile_flags != nullptr) {  // occupied leading rows of every 128-row tile
+      const int sub = B >> 7;
+      for (int i = 0; i < nb * sub; ++i)
+        if (first + i / sub < N) tile_flags[first * sub + i] = min(max(total - i * 128, 0), 128);
+    }
   }
   const int n_cond = mx_conditions ? N + 2 : N + 1;
   const int n_zero = mx_conditions ? n_pad + 2 : n_pad + 1;
@@ -137,7 +142,7 @@ __device__ __forceinline__ int64_t plan_columns(int total, int n_cols, int mode,
 __global__ void __launch_bounds__(1024) group_scan_kernel(int32_t* chunk_counts, int n_chunks, int n_cols, int parts,
                                                           int mode, int T, int B, int N, int mx_conditions,
                                                           int32_t* counts, int64_t* col_base, int32_t* block_to_expert,
-                                                          int32_t* conditions, int32_t* status) {
+                                                          int32_t* conditions, int32_t* tile_flags, int32_t* status) {
   __shared__ int s_sum[1024];  // [parts][1024 / parts]
   const int width = 1024 / parts;
   const int part = threadIdx.x / width, c = threadIdx.x - part * width;
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(1024) group_scan_kernel(int32_t* chunk_counts,
   }
   // the first `width` threads hold the columns' totals; n_cols <= width
   const int64_t base = plan_columns(part == 0 && c < n_cols ? total : 0, n_cols, mode, T, B, N, mx_conditions,
-                                    counts, block_to_expert, conditions, status);
+                                    counts, block_to_expert, conditions, tile_flags, status);
   if (threadIdx.x < static_cast<unsigned>(n_cols)) col_base[threadIdx.x] = base;
 }
 
@@ -229,14 +234,14 @@ __global__ void __launch_bounds__(1024) group_single_chunk_kernel(GroupArgs a, i
                                                                   int64_t out_len, int32_t fill_val, int32_t* out_ids,
                                                                   int32_t* counts, int32_t* block_to_expert,
                                                                   int32_t* conditions, int32_t* inverse_map,
-                                                                  int32_t* status) {
+                                                                  int32_t* tile_flags, int32_t* status) {
   extern __shared__ uint32_t bits[];
   __shared__ int64_t s_base[1024];
   fill_ids(out_ids, out_len, fill_val);
   build_bitmap(a, 0, bits);
   const int c = threadIdx.x;
   s_base[c] = plan_columns(c < a.n_cols ? column_count(bits, c) : 0, a.n_cols, mode, a.T, B, N, mx_conditions, counts,
-                           block_to_expert, conditions, status);
+                           block_to_expert, conditions, tile_flags, status);
   __syncthreads();
   scatter_phase(a, bits, nullptr, s_base, out_len, out_ids, inverse_map);
 }
@@ -294,7 +299,7 @@ __global__ void indexed_flatten_kernel(const int32_t* input, int E, int T, int f
 }
 
 __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_to_expert, const int32_t* conditions,
-                                      int64_t n_pos, int B, int T, int E, int32_t* table) {
+                                      int64_t n_pos, int B, int T, int E, int32_t* table, int32_t* tile_flags) {
   // blocks run up to the first zero condition
   __shared__ int s_n_active;
   const int n_blocks = static_cast<int>(n_pos / B);
@@ -312,7 +317,9 @@ __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_t
     const int t = tpi[p];
     if (t < 0 || t >= T) continue;
     const int e = block_to_expert[b];
-    if (e >= 0 && e < E) table[static_cast<int64_t>(t) * E + e] = static_cast<int32_t>(p);
+    if (e < 0 || e >= E) continue;
+    table[static_cast<int64_t>(t) * E + e] = static_cast<int32_t>(p);
+    if (tile_flags != nullptr) atomicMax(&tile_flags[p >> 7], static_cast<int>(p & 127) + 1);
   }
 }
 
@@ -324,6 +331,7 @@ __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_t
 __global__ void all_expert_setup_kernel(int T, int E_L, int T_pad, int B, int32_t* tpi, int32_t* b2e, int32_t* table,
                                         const void* aff, int aff_dtype, int E, const void* rank_id, int rank_bytes,
                                         const int32_t* selected, int K, float* aff_out) {
+  grid_launch_dependents();
   int64_t first = 0;
   if (rank_id != nullptr)
     first = (rank_bytes == 8 ? *static_cast<const int64_t*>(rank_id) : *static_cast<const int32_t*>(rank_id)) *
@@ -363,7 +371,7 @@ size_t group_ws_bytes(int T, int n_cols) {
 
 int run_grouping(const GroupArgs& a, int mode, int B, int N, int mx_conditions, int64_t out_len, int32_t fill_val,
                  int32_t* out_ids, int32_t* counts, int32_t* block_to_expert, int32_t* conditions, int32_t* inverse_map,
-                 int32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                 int32_t* tile_flags, int32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   B200MOE_REQUIRE(a.T > 0 && a.n_cols > 0 && a.n_cols <= 1024, B200MOE_ERR_INVALID,
                   "grouping: need T > 0 and 0 < columns <= 1024 (got T=%d, columns=%d)", a.T, a.n_cols);
   B200MOE_REQUIRE(workspace_bytes >= group_ws_bytes(a.T, a.n_cols), B200MOE_ERR_WORKSPACE,
@@ -376,7 +384,7 @@ int run_grouping(const GroupArgs& a, int mode, int B, int N, int mx_conditions, 
   const size_t smem = static_cast<size_t>(a.n_cols) * kWords * 4;
   if (n_chunks == 1) {
     group_single_chunk_kernel<<<1, 1024, smem, st>>>(a, mode, B, N, mx_conditions, out_len, fill_val, out_ids, counts,
-                                                     block_to_expert, conditions, inverse_map, status);
+                                                     block_to_expert, conditions, inverse_map, tile_flags, status);
     B200MOE_LAUNCH_OK("group_single_chunk_kernel");
     return B200MOE_OK;
   }
@@ -385,7 +393,7 @@ int run_grouping(const GroupArgs& a, int mode, int B, int N, int mx_conditions, 
   int parts = 1;  // threads per column: as many as 1024 threads allow
   while (parts < 32 && 2 * parts * a.n_cols <= 1024) parts *= 2;
   group_scan_kernel<<<1, 1024, 0, st>>>(chunk_counts, n_chunks, a.n_cols, parts, mode, a.T, B, N, mx_conditions, counts,
-                                        col_base, block_to_expert, conditions, status);
+                                        col_base, block_to_expert, conditions, tile_flags, status);
   B200MOE_LAUNCH_OK("group_scan_kernel");
   group_scatter_kernel<<<n_chunks, kThreads, smem, st>>>(a, chunk_counts, col_base, out_len, out_ids, inverse_map);
   B200MOE_LAUNCH_OK("group_scatter_kernel");
@@ -438,14 +446,16 @@ extern "C" int b200moe_find_nonzero_indices(const void* input, int in_dtype, int
                   n_cols, C_full);
   GroupArgs a{input, B200MOE_ROUTING_MASK, in_dtype, T, C_full, n_cols, 0, col_start_dev};
   return run_grouping(a, 0, 1, 0, 0, static_cast<int64_t>(n_cols) * T, -1, indices, nonzero_counts, nullptr, nullptr,
-                      nullptr, nullptr, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+                      nullptr, nullptr, nullptr, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int b200moe_group_tokens(const void* routing, int routing_mode, int routing_dtype, int T, int E, int K,
+extern "C" int b200moe_group_tokens_tiles(const void* routing, int routing_mode, int routing_dtype, int T, int E, int K,
                                     int B, int N, int skip_token, int mx_conditions, int32_t* token_position_to_id,
                                     int32_t* block_to_expert, int32_t* conditions, int32_t* counts,
-                                    int32_t* inverse_map, int32_t* status, void* workspace, size_t workspace_bytes,
-                                    b200moe_stream_t stream) {
+                                    int32_t* inverse_map, int32_t* tile_flags, int32_t* status, void* workspace,
+                                    size_t workspace_bytes, b200moe_stream_t stream) {
+  B200MOE_REQUIRE(tile_flags == nullptr || B % 128 == 0, B200MOE_ERR_INVALID,
+                  "group_tokens: tile_flags needs a block size that is a multiple of 128, got %d", B);
   B200MOE_REQUIRE(routing && token_position_to_id && block_to_expert && conditions && status && workspace,
                   B200MOE_ERR_INVALID, "group_tokens: null pointer argument");
   B200MOE_REQUIRE(B > 0 && N > 0, B200MOE_ERR_INVALID, "group_tokens: block size and block count must be positive");
@@ -457,8 +467,18 @@ extern "C" int b200moe_group_tokens(const void* routing, int routing_mode, int r
                   "group_tokens: inverse_map needs expert-index routing");
   GroupArgs a{routing, routing_mode, routing_dtype, T, E, E, K, nullptr};
   return run_grouping(a, 1, B, N, mx_conditions, static_cast<int64_t>(N) * B, skip_token ? -1 : T, token_position_to_id,
-                      counts, block_to_expert, conditions, inverse_map, status, workspace, workspace_bytes,
+                      counts, block_to_expert, conditions, inverse_map, tile_flags, status, workspace, workspace_bytes,
                       static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200moe_group_tokens(const void* routing, int routing_mode, int routing_dtype, int T, int E, int K,
+                                    int B, int N, int skip_token, int mx_conditions, int32_t* token_position_to_id,
+                                    int32_t* block_to_expert, int32_t* conditions, int32_t* counts,
+                                    int32_t* inverse_map, int32_t* status, void* workspace, size_t workspace_bytes,
+                                    b200moe_stream_t stream) {
+  return b200moe_group_tokens_tiles(routing, routing_mode, routing_dtype, T, E, K, B, N, skip_token, mx_conditions,
+                                    token_position_to_id, block_to_expert, conditions, counts, inverse_map, nullptr,
+                                    status, workspace, workspace_bytes, stream);
 }
 
 extern "C" int b200moe_cumsum(const void* x, int dtype, int64_t rows, int64_t cols, void* out, b200moe_stream_t stream) {
@@ -486,19 +506,29 @@ extern "C" int b200moe_indexed_flatten(const int32_t* input, int E, int T, int f
   return B200MOE_OK;
 }
 
-extern "C" int b200moe_build_position_table(const int32_t* token_position_to_id, const int32_t* block_to_expert,
+extern "C" int b200moe_build_position_table_tiles(const int32_t* token_position_to_id, const int32_t* block_to_expert,
                                             const int32_t* conditions, int n_blocks, int B, int T, int E,
-                                            int32_t* pos_table, b200moe_stream_t stream) {
+                                            int32_t* pos_table, int32_t* tile_flags, b200moe_stream_t stream) {
+  B200MOE_REQUIRE(tile_flags == nullptr || B % 128 == 0, B200MOE_ERR_INVALID,
+                  "build_position_table: tile_flags needs a block size that is a multiple of 128, got %d", B);
   B200MOE_REQUIRE(token_position_to_id && block_to_expert && pos_table, B200MOE_ERR_INVALID,
                   "build_position_table: null pointer argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   B200MOE_CUDA_OK(cudaMemsetAsync(pos_table, 0xFF, static_cast<size_t>(T) * E * 4, st));
   const int64_t n_pos = static_cast<int64_t>(n_blocks) * B;
+  if (tile_flags != nullptr) B200MOE_CUDA_OK(cudaMemsetAsync(tile_flags, 0, static_cast<size_t>(n_pos / 128) * 4, st));
   const int grid = static_cast<int>(ceil_div64(n_pos, 256) < sm_count() * 8 ? ceil_div64(n_pos, 256) : sm_count() * 8);
   position_table_kernel<<<grid, 256, 0, st>>>(token_position_to_id, block_to_expert, conditions, n_pos, B, T, E,
-                                              pos_table);
+                                              pos_table, tile_flags);
   B200MOE_LAUNCH_OK("position_table_kernel");
   return B200MOE_OK;
+}
+
+extern "C" int b200moe_build_position_table(const int32_t* token_position_to_id, const int32_t* block_to_expert,
+                                            const int32_t* conditions, int n_blocks, int B, int T, int E,
+                                            int32_t* pos_table, b200moe_stream_t stream) {
+  return b200moe_build_position_table_tiles(token_position_to_id, block_to_expert, conditions, n_blocks, B, T, E,
+                                            pos_table, nullptr, stream);
 }
 
 extern "C" int b200moe_all_expert_setup(int T, int E_local, int B, int32_t* token_position_to_id,

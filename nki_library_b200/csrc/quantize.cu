@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) scatter_quantize_kernel(const __nv_bfloat
                                                                int64_t n_pos, int packed, uint8_t* __restrict__ codes,
                                                                uint8_t* __restrict__ sf,
                                                                int32_t* __restrict__ tile_flags) {
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(256) scatter_rows_bf16_kernel(const __nv_bfloa
                                                                 const void* __restrict__ aff, int aff_dtype,
                                                                 __nv_bfloat16* __restrict__ out,
                                                                 int32_t* __restrict__ tile_flags) {
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;

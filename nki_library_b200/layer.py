@@ -91,24 +91,26 @@ class MoELayer:
             self.router_act.value, int(self.pre_norm), int(self.l1), None, _lib.F32, _lib.ptr(self.idx),
             _lib.ptr(self.aff), _lib.F32, self.router_path, _lib.ptr(self.rws), self.rws.numel(), st))
         timed("group_tokens", lambda: _lib.call(
-            "b200moe_group_tokens", _lib.ptr(self.idx), _lib.ROUTING_INDEX, _lib.I32, T, E, K, B, N, 1, 1,
+            "b200moe_group_tokens_tiles", _lib.ptr(self.idx), _lib.ROUTING_INDEX, _lib.I32, T, E, K, B, N, 1, 1,
             _lib.ptr(self.tpi), _lib.ptr(self.b2e), _lib.ptr(self.cond), _lib.ptr(self.counts), _lib.ptr(self.inv),
-            _lib.ptr(self.gstatus), _lib.ptr(self.gws), self.gws.numel(), st))
+            _lib.ptr(ws.tile_flags), _lib.ptr(self.gstatus), _lib.ptr(self.gws), self.gws.numel(), st))
         # token-major: each row is read and quantised once and stored to its K positions
         timed("gather_quantize", lambda: _lib.call(
             "b200moe_scatter_quantize_mxfp8", _lib.ptr(hidden), T, H, _lib.ptr(self.inv), K, N * B,
-            int(w.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(ws.tile_flags), st))
+            int(w.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), None, st))
         nan = float("nan")
         timed("gemm1_swiglu", lambda: _lib.call(
             "b200moe_grouped_gemm1_swiglu", _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(w.w1), _lib.ptr(w.w1_sf), w.w_format,
             _lib.ptr(w.bias_gu), _lib.ptr(self.b2e), _lib.ptr(self.cond), _lib.ptr(ws.tile_flags), N, B, E, H, I,
             self.act_fn.value, nan, nan, nan, nan, _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(ws.status) + 4,
-            self.gemm_variant, None if self.clock_probe is None else _lib.ptr(self.clock_probe[0:]), st))
+            self.gemm_variant | _lib.GEMM_CHAINED,
+            None if self.clock_probe is None else _lib.ptr(self.clock_probe[0:]), st))
         timed("gemm2_scale", lambda: _lib.call(
             "b200moe_grouped_gemm2_scale", _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(w.w2), _lib.ptr(w.w2_sf), w.w_format,
             _lib.ptr(w.bias_d), _lib.ptr(self.b2e), _lib.ptr(self.cond), _lib.ptr(ws.tile_flags), _lib.ptr(self.tpi),
             T, N, B, E, H, I, _lib.ptr(self.aff), _lib.F32, 0, _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8,
-            self.gemm_variant, None if self.clock_probe is None else _lib.ptr(self.clock_probe[2:]), st))
+            self.gemm_variant | _lib.GEMM_CHAINED,
+            None if self.clock_probe is None else _lib.ptr(self.clock_probe[2:]), st))
         timed("combine", lambda: _lib.call(
             "b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(self.inv), T, K, H, _lib.ptr(out), st))
         return out

@@ -57,7 +57,7 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
                affinities: Optional[torch.Tensor], table: torch.Tensor, out: torch.Tensor, act_fn: int = 0,
                gate_clamp=(None, None), up_clamp=(None, None), impl: int = 0, check_status: bool = False,
                workspace: Optional[BlockWorkspace] = None, aff_per_row: bool = False,
-               timers: Optional[dict] = None, prequantized: bool = False) -> torch.Tensor:
+               timers: Optional[dict] = None, prequantized: bool = False, flags_ready: bool = False) -> torch.Tensor:
     """Run the four kernels.  ``table [rows_out, n_cand]`` lists, per output row (= token), the positions that
     hold it (negative = none): the quantiser stores the token's row there and the combine sums those rows.
 
@@ -66,7 +66,8 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
     ``token * E + expert`` (fp32 or bf16), a per-row vector addressed ``token``
     when ``aff_per_row``, or None.  ``out`` bf16 ``[rows_out, H]``.  With ``prequantized`` the caller has already
     filled ``workspace.xq / x_sf / tile_flags`` for this ``table`` (the fused RMSNorm + quantise kernel) and the
-    quantise launch is skipped.
+    quantise launch is skipped.  ``flags_ready``: ``workspace.tile_flags`` of these blocks was filled by an earlier
+    launch than the one directly in front, which lets the gate/up contraction start while the quantiser drains.
     """
     E, H, I = weights.E, weights.H, weights.I
     n_blocks = block_to_expert.numel()
@@ -90,19 +91,19 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
     if not prequantized:
         _lib.call("b200moe_scatter_quantize_mxfp8", _lib.ptr(hidden), min(hidden_rows, table.shape[0]), H, _lib.ptr(table),
                   table.shape[1], n_pos, int(weights.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf),
-                  _lib.ptr(ws.tile_flags), st)
+                  None if flags_ready else _lib.ptr(ws.tile_flags), st)
     mark("t1")
     _lib.call("b200moe_grouped_gemm1_swiglu", _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(weights.w1),
               _lib.ptr(weights.w1_sf), weights.w_format, _lib.ptr(weights.bias_gu), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), n_blocks, block_size, E, H, I, act_fn, _clamp(gate_clamp[0]),
               _clamp(gate_clamp[1]), _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.mq), _lib.ptr(ws.m_sf),
-              _lib.ptr(ws.status) + 4, impl, None, st)
+              _lib.ptr(ws.status) + 4, impl | (_lib.GEMM_CHAINED if flags_ready else 0), None, st)
     mark("t2")
     _lib.call("b200moe_grouped_gemm2_scale", _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(weights.w2),
               _lib.ptr(weights.w2_sf), weights.w_format, _lib.ptr(weights.bias_d), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), _lib.ptr(token_position_to_id), hidden_rows, n_blocks, block_size, E, H, I,
               _lib.ptr(affinities), _lib.F32 if affinities is None else _lib.dtype_code(affinities),
-              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8, impl, None, st)
+              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8, impl | _lib.GEMM_CHAINED, None, st)
     mark("t3")
     _lib.call("b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(table), out.shape[0], table.shape[1], H, _lib.ptr(out), st)
     if check_status:
@@ -125,11 +126,22 @@ class DenseWorkspace:
 _dense_workspaces: dict = {}
 
 
+def get_dense_workspace(n_pos: int, H: int, I: int, device) -> DenseWorkspace:
+    key = (n_pos, H, I, str(device))
+    ws = _dense_workspaces.get(key)
+    if ws is None:
+        if len(_dense_workspaces) > 4:
+            _dense_workspaces.clear()
+        ws = _dense_workspaces[key] = DenseWorkspace(n_pos, H, I, device)
+    return ws
+
+
 def run_blocks_dense(hidden: torch.Tensor, hidden_rows: int, weights, token_position_to_id: torch.Tensor,
                      block_to_expert: torch.Tensor, conditions: Optional[torch.Tensor], block_size: int,
                      affinities: Optional[torch.Tensor], table: torch.Tensor, out: torch.Tensor, act_fn: int = 0,
                      gate_clamp=(None, None), up_clamp=(None, None), impl: int = 0, check_status: bool = False,
-                     pre_scale: bool = False) -> torch.Tensor:
+                     pre_scale: bool = False, workspace: Optional["DenseWorkspace"] = None,
+                     flags_ready: bool = False) -> torch.Tensor:
     """The four launches of the dense variants: row scatter (x affinity when ``pre_scale``) -> gate/up contraction
     + bias + clamp + act(gate) * up -> down contraction + bias (x affinity unless ``pre_scale``) -> combine.
     Arguments as :func:`run_blocks`; ``weights`` is a :class:`~nki_library_b200.weights.DenseExpertWeights`."""
@@ -140,26 +152,23 @@ def run_blocks_dense(hidden: torch.Tensor, hidden_rows: int, weights, token_posi
     _lib.kernel_assert(token_position_to_id.numel() == n_pos, "token_position_to_id must hold N * block_size ids")
     _lib.kernel_assert(hidden.dtype == torch.bfloat16 and hidden.shape[1] == H and hidden.is_contiguous(),
                        "hidden_states must be contiguous bf16 [rows, H]")
-    key = (n_pos, H, I, str(hidden.device))
-    ws = _dense_workspaces.get(key)
-    if ws is None:
-        if len(_dense_workspaces) > 4:
-            _dense_workspaces.clear()
-        ws = _dense_workspaces[key] = DenseWorkspace(n_pos, H, I, hidden.device)
+    ws = workspace or get_dense_workspace(n_pos, H, I, hidden.device)
     st = _lib.stream_ptr()
     aff_code = _lib.F32 if affinities is None else _lib.dtype_code(affinities)
     _lib.call("b200moe_scatter_rows_bf16", _lib.ptr(hidden), min(hidden_rows, table.shape[0]), H, _lib.ptr(table),
               table.shape[1], n_pos, _lib.ptr(block_to_expert), block_size, E,
-              _lib.ptr(affinities) if pre_scale else None, aff_code, _lib.ptr(ws.x_pos), _lib.ptr(ws.tile_flags), st)
+              _lib.ptr(affinities) if pre_scale else None, aff_code, _lib.ptr(ws.x_pos),
+              None if flags_ready else _lib.ptr(ws.tile_flags), st)
     _lib.call("b200moe_dense_gemm1_swiglu", _lib.ptr(ws.x_pos), _lib.ptr(weights.w1), _lib.ptr(weights.scale_gu),
               _lib.ptr(weights.bias_gu), _lib.ptr(block_to_expert), _lib.ptr(conditions), _lib.ptr(ws.tile_flags),
               n_blocks, block_size, E, H, I, act_fn, _clamp(gate_clamp[0]), _clamp(gate_clamp[1]),
-              _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.m), _lib.ptr(ws.status) + 4, impl, st)
+              _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.m), _lib.ptr(ws.status) + 4,
+              impl | (_lib.GEMM_CHAINED if flags_ready else 0), st)
     _lib.call("b200moe_dense_gemm2_scale", _lib.ptr(ws.m), _lib.ptr(weights.w2), _lib.ptr(weights.scale_d),
               _lib.ptr(weights.bias_d), _lib.ptr(block_to_expert), _lib.ptr(conditions), _lib.ptr(ws.tile_flags),
               _lib.ptr(token_position_to_id), hidden_rows, n_blocks, block_size, E, H, I,
               None if pre_scale else _lib.ptr(affinities), aff_code, 0, _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8,
-              impl, st)
+              impl | _lib.GEMM_CHAINED, st)
     _lib.call("b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(table), out.shape[0], table.shape[1], H, _lib.ptr(out), st)
     if check_status:
         s = ws.status.cpu().tolist()

@@ -188,3 +188,24 @@ def test_router_narrow_and_odd_widths(E):
     p = torch.softmax(logits, 1).gather(1, idx.long())
     want = torch.zeros_like(aff).scatter_(1, idx.long(), p / p.sum(1, keepdim=True))
     assert bool(((aff - want).abs() <= 1e-5 * want + 1e-12).all())
+
+
+@pytest.mark.parametrize("T,E,K,B", [(3, 128, 8, 128), (256, 5, 2, 256), (3000, 40, 4, 128), (3000, 3, 1, 512)])
+def test_tile_flags_from_bookkeeping(T, E, K, B):
+    """The occupied rows per 128 positions, from the grouping and from the position table, are what the quantiser's
+    stores say."""
+    import nki_library_b200 as m
+    L = _lib()
+    idx = torch.rand((T, E), device="cuda", generator=_gen(T + E)).topk(K, dim=1).indices.to(torch.int32)
+    N = m.get_n_blocks(T, K, E, B)
+    flags = torch.full((N * B // 128,), 77, dtype=torch.int32, device="cuda")
+    g = m.moe_group_tokens(idx, E, B, N, top_k=K, _tile_flags=flags)
+    rows = torch.arange(128, device="cuda") + 1
+    want = ((g["token_position_to_id"].view(-1, 128) >= 0) * rows).amax(1).int()
+    assert torch.equal(flags, want)
+    table = torch.empty((T, E), dtype=torch.int32, device="cuda")
+    flags.fill_(77)
+    L.call("b200moe_build_position_table_tiles", L.ptr(g["token_position_to_id"]), L.ptr(g["block_to_expert"]),
+           L.ptr(g["conditions"]), N, B, T, E, L.ptr(table), L.ptr(flags), L.stream_ptr())
+    assert torch.equal(flags, want)
+    assert torch.equal(table.gather(1, idx.long()), g["inverse_map"])
