@@ -209,3 +209,35 @@ def test_tile_flags_from_bookkeeping(T, E, K, B):
            L.ptr(g["conditions"]), N, B, T, E, L.ptr(table), L.ptr(flags), L.stream_ptr())
     assert torch.equal(flags, want)
     assert torch.equal(table.gather(1, idx.long()), g["inverse_map"])
+
+
+@pytest.mark.parametrize("act", ["SOFTMAX", "SIGMOID"])
+@pytest.mark.parametrize("mode", ["norm", "pre", "post"])
+@pytest.mark.parametrize("E,k", [(8, 8), (33, 3), (128, 8), (512, 1)])
+def test_router_winner_lanes(act, mode, E, k):
+    """Winners are activated and written by their own lanes: every pipeline, ties, -0 and -inf logits (from the bias)."""
+    import nki_library_b200 as m
+    T, H = 19, 256
+    x = torch.randn((T, H), device="cuda", generator=_gen(13)).to(torch.bfloat16)
+    x[0] = 0  # all logits are the bias: ties
+    w = (torch.randn((H, E), device="cuda", generator=_gen(14)) * 0.1).to(torch.bfloat16)
+    bias = torch.zeros((E,), device="cuda", dtype=torch.bfloat16)
+    bias[1::3] = -0.0
+    bias[E - 1] = float("-inf")
+    logits, aff = torch.empty((T, E), device="cuda"), torch.full((T, E), 9.0, device="cuda")
+    idx = torch.empty((T, k), dtype=torch.int32, device="cuda")
+    m.router_topk(x, w, bias, logits, aff, idx, m.RouterActFnType[act], k, 1, 0, router_pre_norm=mode != "post",
+                  norm_topk_prob=mode == "norm", use_indirect_dma_scatter=True)
+    order = torch.sort(logits + 0.0, dim=1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(idx.long(), order)
+    top = logits.gather(1, order).double()
+    if act == "SIGMOID":
+        val, full = torch.sigmoid(top), torch.sigmoid(logits.double())
+    else:
+        full = torch.softmax(logits.double(), 1)
+        val = full.gather(1, order) if mode != "post" else torch.softmax(top, 1)
+    if mode == "norm":
+        val = val / val.sum(1, keepdim=True)
+    want = full if mode == "pre" else torch.zeros_like(full).scatter_(1, order, val)
+    # a handful of fp32 operations per value, exponents of up to ~10: 1e-5 relative
+    assert bool(((aff.double() - want).abs() <= 1e-5 * want + 1e-12).all())
