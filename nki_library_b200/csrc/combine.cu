@@ -18,6 +18,7 @@ __global__ void __launch_bounds__(128) combine_kernel(const __nv_bfloat16* __res
                                                       __nv_bfloat16* __restrict__ out) {
   extern __shared__ int32_t s_rows[];  // n_cand entries: every candidate may be valid (all-expert decode)
   __shared__ int s_n;
+  grid_enter(y_pos, table);
   const int t = blockIdx.x;
   if (threadIdx.x < 32) {
     int base = 0;
@@ -81,8 +82,9 @@ extern "C" int b200moe_combine(const void* y_pos_bf16, const int32_t* table, int
                   kMaxCandidates, n_cand);
   // a CTA covers 1024 columns at a time: one per token once the tokens alone give every SM several
   const int col_ctas = T >= 8 * sm_count() ? 1 : (H + 1023) / 1024;
-  combine_kernel<<<dim3(T, col_ctas), 128, static_cast<size_t>(n_cand) * sizeof(int32_t), static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(y_pos_bf16), table, T, n_cand, H, static_cast<__nv_bfloat16*>(out_bf16));
+  B200MOE_CUDA_OK(launch_overlapped(combine_kernel, dim3(T, col_ctas), 128, static_cast<size_t>(n_cand) * sizeof(int32_t),
+                                    static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(y_pos_bf16), table,
+                                    T, n_cand, H, static_cast<__nv_bfloat16*>(out_bf16)));
   B200MOE_LAUNCH_OK("combine_kernel");
   return B200MOE_OK;
 }

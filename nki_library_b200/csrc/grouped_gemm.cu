@@ -106,7 +106,7 @@ __device__ __forceinline__ int token_tiles(const GemmParams& p, int rows) {
 //
 // Everything read from global memory here is fetched at once into `scratch` (shared memory the pipeline will use
 // later, `scratch_ints` long; larger problems read global memory again): the prologue costs one memory latency, which
-// is what a decode launch of a few tens of microseconds notices.
+// is what a decode launch of a few tens of microseconds notices.  (A chained launch reads before it waits: past L1.)
 template <int CTAS, int EPI>
 __device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n_units, int* scratch, int scratch_ints,
                                             int ring_bytes, int slab_fixed_bytes, int max_stages) {
@@ -119,14 +119,14 @@ __device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n
   const int32_t* flags = p.tile_flags;
   const bool staged = p.n_blocks + p.m_tiles_total <= scratch_ints;
   for (int b = tid; b < p.n_blocks; b += nthr) {
-    const int e = staged ? p.block_to_expert[b] : 0;
-    const int run = p.conditions != nullptr ? p.conditions[b] : 1;
+    const int e = staged ? __ldcg(p.block_to_expert + b) : 0;
+    const int run = p.conditions != nullptr ? __ldcg(p.conditions + b) : 1;
     if (staged) scratch[b] = e;
     if (run == 0) atomicMin(&s.n_active, b);
   }
   if (staged) {
     if (p.tile_flags != nullptr) {
-      for (int t = tid; t < p.m_tiles_total; t += nthr) scratch[p.n_blocks + t] = p.tile_flags[t];
+      for (int t = tid; t < p.m_tiles_total; t += nthr) scratch[p.n_blocks + t] = __ldcg(p.tile_flags + t);
       flags = scratch + p.n_blocks;
     }
     b2e = scratch;
@@ -255,7 +255,7 @@ __device__ __forceinline__ TileRec decode_tile(const GemmParams& p, const Sched&
     const int rows = s.rows[e];
     if (rows < 0) {
       row0 = s.first_row[e] + t * 128;
-      n = p.tile_flags[row0 >> 7];
+      n = __ldcg(p.tile_flags + (row0 >> 7));
       if (n > p.max_n) n = p.max_n;  // (max_n is at least 128)
     } else {
       const int width = round_up((rows + cnt - 1) / cnt, kStepN);
@@ -272,9 +272,9 @@ __device__ __forceinline__ TileRec decode_tile(const GemmParams& p, const Sched&
     const int within = tile - g * per_group;
     const int m_tile = first + within % gs;
     w_tile = within / gs;
-    e = p.block_to_expert[m_tile / (p.B >> 7)];
+    e = __ldcg(p.block_to_expert + m_tile / (p.B >> 7));
     row0 = m_tile * 128;
-    n = (e < 0 || e >= p.E) ? 0 : (p.tile_flags ? p.tile_flags[m_tile] : 128);
+    n = (e < 0 || e >= p.E) ? 0 : (p.tile_flags ? __ldcg(p.tile_flags + m_tile) : 128);
   }
   const int h = cut ? s.h / s.parts : s.h;
   const int w_row0 = w_tile * s.h + sub_part * h;
@@ -503,7 +503,7 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
       // weights do not depend on the launch in front, the token rows and their scales do
       if (p.chained && warp != 0) grid_wait();
       // not before the launch in front is complete: the next one reads more than this one before it waits
-      if (EPI == 0 && warp == 3) grid_launch_dependents();
+      if (warp == 3) grid_launch_dependents();
       for (int tile = unit, it = 0; tile < total_tiles && ok; tile += n_units, ++it) {
         const TileRec r = fetch_tile<CTAS>(p, sched, tile_table, it, tile);
         if (r.shape == 0 || (KIND != 0 && warp == 2)) continue;
@@ -717,7 +717,7 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
           float aff = 1.0f;
           if (col < n) {
             const int pos = r.row0 + col;
-            const int tok = p.tpi ? p.tpi[pos] : pos;
+            const int tok = p.tpi ? __ldcg(p.tpi + pos) : pos;
             if (tok >= 0 && tok < p.hidden_rows) {
               dst = pos;
               if (p.row_src != nullptr) {
@@ -725,8 +725,8 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
                 if ((dst >> 24) >= 8 || (dst & 0xffffff) >= p.peer_rows || p.peer_out[dst >> 24] == nullptr) dst = -1;
               }
               if (p.aff != nullptr)
-                aff = load_as_float(p.aff, p.aff_per_row ? static_cast<int64_t>(tok) : static_cast<int64_t>(tok) * p.E + r.expert,
-                                    p.aff_dtype);
+                aff = load_as_float<true>(p.aff, p.aff_per_row ? static_cast<int64_t>(tok) : static_cast<int64_t>(tok) * p.E + r.expert,
+                                          p.aff_dtype);
             }
           }
           tok_aff[tg] = aff;
@@ -1143,7 +1143,6 @@ int launch_tc(const WeightMaps& wm, const TokenMaps& xm, const CUtensorMap& sfw,
   // from the last CTA's end to the first one's start, and 8 to 10 more to the first slab in shared memory.
   // 64-token decode of 8 experts of 4096 x 14336: 274 -> 264 us, 16 tokens on 128 experts of 4096 x 1536, top-8,
   // captured: 285 -> 273 us.
-  // @P_CHAIN@
   cudaLaunchAttribute attr[2];
   if (CTAS == 2) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;

@@ -77,6 +77,7 @@ __device__ __forceinline__ void fill_ids(int32_t* ids, int64_t n, int32_t value)
 __global__ void __launch_bounds__(kThreads) group_count_kernel(GroupArgs a, int32_t* chunk_counts, int32_t* fill_ptr,
                                                                int64_t fill_n, int32_t fill_val) {
   extern __shared__ uint32_t bits[];
+  grid_enter();
   fill_ids(fill_ptr, fill_n, fill_val);
   build_bitmap(a, blockIdx.x, bits);
   for (int c = threadIdx.x; c < a.n_cols; c += blockDim.x)
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(1024) group_scan_kernel(int32_t* chunk_counts,
                                                           int32_t* counts, int64_t* col_base, int32_t* block_to_expert,
                                                           int32_t* conditions, int32_t* tile_flags, int32_t* status) {
   __shared__ int s_sum[1024];  // [parts][1024 / parts]
+  grid_enter();
   const int width = 1024 / parts;
   const int part = threadIdx.x / width, c = threadIdx.x - part * width;
   const int span = (n_chunks + parts - 1) / parts;
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(kThreads) group_scatter_kernel(GroupArgs a, co
                                                                  const int64_t* col_base, int64_t out_len,
                                                                  int32_t* out_ids, int32_t* inverse_map) {
   extern __shared__ uint32_t bits[];
+  grid_enter();
   build_bitmap(a, blockIdx.x, bits);
   scatter_phase(a, bits, chunk_prefix, col_base, out_len, out_ids, inverse_map);
 }
@@ -237,6 +240,7 @@ __global__ void __launch_bounds__(1024) group_single_chunk_kernel(GroupArgs a, i
                                                                   int32_t* tile_flags, int32_t* status) {
   extern __shared__ uint32_t bits[];
   __shared__ int64_t s_base[1024];
+  grid_enter();
   fill_ids(out_ids, out_len, fill_val);
   build_bitmap(a, 0, bits);
   const int c = threadIdx.x;
@@ -302,6 +306,7 @@ __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_t
                                       int64_t n_pos, int B, int T, int E, int32_t* table, int32_t* tile_flags) {
   // blocks run up to the first zero condition
   __shared__ int s_n_active;
+  grid_enter();
   const int n_blocks = static_cast<int>(n_pos / B);
   if (threadIdx.x == 0) s_n_active = n_blocks;
   __syncthreads();
@@ -331,7 +336,7 @@ __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_t
 __global__ void all_expert_setup_kernel(int T, int E_L, int T_pad, int B, int32_t* tpi, int32_t* b2e, int32_t* table,
                                         const void* aff, int aff_dtype, int E, const void* rank_id, int rank_bytes,
                                         const int32_t* selected, int K, float* aff_out) {
-  grid_launch_dependents();
+  grid_enter();
   int64_t first = 0;
   if (rank_id != nullptr)
     first = (rank_bytes == 8 ? *static_cast<const int64_t*>(rank_id) : *static_cast<const int32_t*>(rank_id)) *
@@ -383,19 +388,23 @@ int run_grouping(const GroupArgs& a, int mode, int B, int N, int mx_conditions, 
                                                  ((static_cast<size_t>(n_chunks) * a.n_cols * 4 + 255) / 256) * 256);
   const size_t smem = static_cast<size_t>(a.n_cols) * kWords * 4;
   if (n_chunks == 1) {
-    group_single_chunk_kernel<<<1, 1024, smem, st>>>(a, mode, B, N, mx_conditions, out_len, fill_val, out_ids, counts,
-                                                     block_to_expert, conditions, inverse_map, tile_flags, status);
+    B200MOE_CUDA_OK(launch_overlapped(group_single_chunk_kernel, dim3(1), 1024, smem, st, a, mode, B, N, mx_conditions,
+                                      out_len, fill_val, out_ids, counts, block_to_expert, conditions, inverse_map,
+                                      tile_flags, status));
     B200MOE_LAUNCH_OK("group_single_chunk_kernel");
     return B200MOE_OK;
   }
-  group_count_kernel<<<n_chunks, kThreads, smem, st>>>(a, chunk_counts, out_ids, out_len, fill_val);
+  B200MOE_CUDA_OK(launch_overlapped(group_count_kernel, dim3(n_chunks), kThreads, smem, st, a, chunk_counts, out_ids,
+                                    out_len, fill_val));
   B200MOE_LAUNCH_OK("group_count_kernel");
   int parts = 1;  // threads per column: as many as 1024 threads allow
   while (parts < 32 && 2 * parts * a.n_cols <= 1024) parts *= 2;
-  group_scan_kernel<<<1, 1024, 0, st>>>(chunk_counts, n_chunks, a.n_cols, parts, mode, a.T, B, N, mx_conditions, counts,
-                                        col_base, block_to_expert, conditions, tile_flags, status);
+  B200MOE_CUDA_OK(launch_overlapped(group_scan_kernel, dim3(1), 1024, 0, st, chunk_counts, n_chunks, a.n_cols, parts, mode,
+                                    a.T, B, N, mx_conditions, counts,
+                                    col_base, block_to_expert, conditions, tile_flags, status));
   B200MOE_LAUNCH_OK("group_scan_kernel");
-  group_scatter_kernel<<<n_chunks, kThreads, smem, st>>>(a, chunk_counts, col_base, out_len, out_ids, inverse_map);
+  B200MOE_CUDA_OK(launch_overlapped(group_scatter_kernel, dim3(n_chunks), kThreads, smem, st, a, chunk_counts, col_base,
+                                    out_len, out_ids, inverse_map));
   B200MOE_LAUNCH_OK("group_scatter_kernel");
   return B200MOE_OK;
 }
@@ -518,8 +527,8 @@ extern "C" int b200moe_build_position_table_tiles(const int32_t* token_position_
   const int64_t n_pos = static_cast<int64_t>(n_blocks) * B;
   if (tile_flags != nullptr) B200MOE_CUDA_OK(cudaMemsetAsync(tile_flags, 0, static_cast<size_t>(n_pos / 128) * 4, st));
   const int grid = static_cast<int>(ceil_div64(n_pos, 256) < sm_count() * 8 ? ceil_div64(n_pos, 256) : sm_count() * 8);
-  position_table_kernel<<<grid, 256, 0, st>>>(token_position_to_id, block_to_expert, conditions, n_pos, B, T, E,
-                                              pos_table, tile_flags);
+  B200MOE_CUDA_OK(launch_overlapped(position_table_kernel, dim3(grid), 256, 0, st, token_position_to_id, block_to_expert,
+                                    conditions, n_pos, B, T, E, pos_table, tile_flags));
   B200MOE_LAUNCH_OK("position_table_kernel");
   return B200MOE_OK;
 }
@@ -551,9 +560,10 @@ extern "C" int b200moe_all_expert_setup(int T, int E_local, int B, int32_t* toke
   const int64_t n_pos = T_pad * E_local;
   B200MOE_REQUIRE(n_pos < (1LL << 31), B200MOE_ERR_INVALID, "all_expert_setup: more than 2^31 positions");
   const int64_t cap = static_cast<int64_t>(sm_count()) * 8, want = ceil_div64(n_pos, 256);
-  all_expert_setup_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      T, E_local, static_cast<int>(T_pad), B, token_position_to_id, block_to_expert, pos_table, affinities, aff_dtype, E,
-      rank_id, rank_bytes, expert_index, K, local_affinities);
+  B200MOE_CUDA_OK(launch_overlapped(all_expert_setup_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), 256, 0,
+                                    static_cast<cudaStream_t>(stream), T, E_local, static_cast<int>(T_pad), B,
+                                    token_position_to_id, block_to_expert, pos_table, affinities, aff_dtype, E, rank_id,
+                                    rank_bytes, expert_index, K, local_affinities));
   B200MOE_LAUNCH_OK("all_expert_setup_kernel");
   return B200MOE_OK;
 }

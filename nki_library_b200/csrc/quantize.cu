@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) scatter_quantize_kernel(const __nv_bfloat
                                                                int64_t n_pos, int packed, uint8_t* __restrict__ codes,
                                                                uint8_t* __restrict__ sf,
                                                                int32_t* __restrict__ tile_flags) {
-  grid_launch_dependents();
+  grid_enter(hidden, inverse_map);
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) scatter_rows_bf16_kernel(const __nv_bfloa
                                                                 const void* __restrict__ aff, int aff_dtype,
                                                                 __nv_bfloat16* __restrict__ out,
                                                                 int32_t* __restrict__ tile_flags) {
-  grid_launch_dependents();
+  grid_enter(hidden, table, block_to_expert, aff);
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -396,9 +396,9 @@ extern "C" int b200moe_scatter_quantize_mxfp8(const void* hidden_bf16, int T, in
   if (tile_flags != nullptr)
     B200MOE_CUDA_OK(cudaMemsetAsync(tile_flags, 0, static_cast<size_t>(ceil_div64(n_pos, 128)) * 4, st));
   const dim3 grid(static_cast<unsigned>((T + 7) / 8), static_cast<unsigned>((H + 1023) / 1024));
-  scatter_quantize_kernel<<<grid, 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(hidden_bf16), T, H, inverse_map, K, n_pos, h_packed_order, codes, sf_atoms,
-      tile_flags);
+  B200MOE_CUDA_OK(launch_overlapped(scatter_quantize_kernel, grid, 256, 0, st,
+                                    static_cast<const __nv_bfloat16*>(hidden_bf16), T, H, inverse_map, K, n_pos,
+                                    h_packed_order, codes, sf_atoms, tile_flags));
   B200MOE_LAUNCH_OK("scatter_quantize_kernel");
   return B200MOE_OK;
 }
@@ -417,9 +417,10 @@ extern "C" int b200moe_scatter_rows_bf16(const void* hidden_bf16, int T, int H, 
   if (tile_flags != nullptr)
     B200MOE_CUDA_OK(cudaMemsetAsync(tile_flags, 0, static_cast<size_t>(ceil_div64(n_pos, 128)) * 4, st));
   const dim3 grid(static_cast<unsigned>((T + 7) / 8), static_cast<unsigned>((H + 1023) / 1024));
-  scatter_rows_bf16_kernel<<<grid, 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(hidden_bf16), T, H, table, K, n_pos, block_to_expert, B, E,
-      pre_scale_affinities, aff_dtype, static_cast<__nv_bfloat16*>(out_bf16), tile_flags);
+  B200MOE_CUDA_OK(launch_overlapped(scatter_rows_bf16_kernel, grid, 256, 0, st,
+                                    static_cast<const __nv_bfloat16*>(hidden_bf16), T, H, table, K, n_pos,
+                                    block_to_expert, B, E, pre_scale_affinities, aff_dtype,
+                                    static_cast<__nv_bfloat16*>(out_bf16), tile_flags));
   B200MOE_LAUNCH_OK("scatter_rows_bf16_kernel");
   return B200MOE_OK;
 }

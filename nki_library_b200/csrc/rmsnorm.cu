@@ -105,6 +105,7 @@ __device__ __forceinline__ bool rows_aligned(const NormArgs& a) {
 }
 
 __global__ void __launch_bounds__(512) rmsnorm_kernel(NormArgs a) {
+  grid_enter();
   const int64_t base = static_cast<int64_t>(blockIdx.x) * a.H;
   const bool vec = rows_aligned(a);
   const float rinv = row_rinv(a, base, vec);
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(512) rmsnorm_quantize_kernel(NormArgs a, const
                                                                int64_t n_pos, int packed, uint8_t* __restrict__ codes,
                                                                uint8_t* __restrict__ sf,
                                                                int32_t* __restrict__ tile_flags) {
+  grid_enter(table);
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x, H = a.H;
   const int64_t base = static_cast<int64_t>(t) * H;
@@ -195,7 +197,8 @@ extern "C" int b200moe_rmsnorm_quantize_mxfp8(const void* inp_bf16, const void* 
   const NormArgs a{static_cast<const __nv_bfloat16*>(inp_bf16), static_cast<const __nv_bfloat16*>(residual_bf16), gamma,
                    gamma_dtype, H, inv_count, eps, static_cast<__nv_bfloat16*>(out_bf16),
                    static_cast<__nv_bfloat16*>(residual_out_bf16)};
-  rmsnorm_quantize_kernel<<<T, norm_threads(H), 0, st>>>(a, table, K, n_pos, h_packed_order, codes, sf_atoms, tile_flags);
+  B200MOE_CUDA_OK(launch_overlapped(rmsnorm_quantize_kernel, dim3(T), norm_threads(H), 0, st, a, table, K, n_pos,
+                                    h_packed_order, codes, sf_atoms, tile_flags));
   B200MOE_LAUNCH_OK("rmsnorm_quantize_kernel");
   return B200MOE_OK;
 }
@@ -210,7 +213,7 @@ extern "C" int b200moe_rmsnorm(const void* inp_bf16, const void* residual_bf16, 
   const NormArgs a{static_cast<const __nv_bfloat16*>(inp_bf16), static_cast<const __nv_bfloat16*>(residual_bf16), gamma,
                    gamma_dtype, H, inv_count, eps, static_cast<__nv_bfloat16*>(out_bf16),
                    static_cast<__nv_bfloat16*>(residual_out_bf16)};
-  rmsnorm_kernel<<<T, norm_threads(H), 0, static_cast<cudaStream_t>(stream)>>>(a);
+  B200MOE_CUDA_OK(launch_overlapped(rmsnorm_kernel, dim3(T), norm_threads(H), 0, static_cast<cudaStream_t>(stream), a));
   B200MOE_LAUNCH_OK("rmsnorm_kernel");
   return B200MOE_OK;
 }

@@ -66,6 +66,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 // w slab: [kKC][EN + pad].
 __global__ void __launch_bounds__(256) router_logits_kernel(LogitArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_enter();
   const int TM = 16 * a.mw, EN = 64 * a.nw;
   const int x_stride = a.x_is_TH ? (kKC + kXPad) : (TM + kXPad);
   const int x_rows = a.x_is_TH ? TM : kKC;
@@ -216,6 +217,7 @@ struct RankArgs {
 // NPL = experts per lane (E <= 32 * NPL); instantiated for 1, 2, 4, 8, 16 so small expert counts do not pay for 512.
 template <int NPL>
 __global__ void __launch_bounds__(256) router_rank_kernel(RankArgs a) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= a.T) return;
@@ -437,18 +439,18 @@ extern "C" int b200moe_router_topk(const void* x, int x_is_TH, const void* w, co
     LogitArgs la{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), x_is_TH, T, H, E,
                  p.mw, p.nw, p.h_per_split, p.stages, static_cast<float*>(workspace), status};
     dim3 grid((T + p.tm - 1) / p.tm, p.splits);
-    router_logits_kernel<<<grid, 256, p.smem, st>>>(la);
+    B200MOE_CUDA_OK(launch_overlapped(router_logits_kernel, grid, 256, p.smem, st, la));
     B200MOE_LAUNCH_OK("router_logits_kernel");
   }
   RankArgs ra{partial, splits, static_cast<const __nv_bfloat16*>(w_bias), T, E, k,
               act_fn, router_pre_norm, norm_topk_prob, router_logits, logits_dtype, expert_index, expert_affinities,
               aff_dtype};
   const dim3 rgrid((T + 7) / 8);
-  if (E <= 32) router_rank_kernel<1><<<rgrid, 256, 0, st>>>(ra);
-  else if (E <= 64) router_rank_kernel<2><<<rgrid, 256, 0, st>>>(ra);
-  else if (E <= 128) router_rank_kernel<4><<<rgrid, 256, 0, st>>>(ra);
-  else if (E <= 256) router_rank_kernel<8><<<rgrid, 256, 0, st>>>(ra);
-  else router_rank_kernel<16><<<rgrid, 256, 0, st>>>(ra);
+  if (E <= 32) B200MOE_CUDA_OK(launch_overlapped(router_rank_kernel<1>, rgrid, 256, 0, st, ra));
+  else if (E <= 64) B200MOE_CUDA_OK(launch_overlapped(router_rank_kernel<2>, rgrid, 256, 0, st, ra));
+  else if (E <= 128) B200MOE_CUDA_OK(launch_overlapped(router_rank_kernel<4>, rgrid, 256, 0, st, ra));
+  else if (E <= 256) B200MOE_CUDA_OK(launch_overlapped(router_rank_kernel<8>, rgrid, 256, 0, st, ra));
+  else B200MOE_CUDA_OK(launch_overlapped(router_rank_kernel<16>, rgrid, 256, 0, st, ra));
   B200MOE_LAUNCH_OK("router_rank_kernel");
   return B200MOE_OK;
 }
