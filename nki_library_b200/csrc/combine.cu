@@ -8,11 +8,12 @@ namespace {
 
 constexpr int kMaxCandidates = 8192;  // table width limit: the row list of one token lives in shared memory
 
-// Bound by the y_pos rows it reads (n_cand of them per token, 32768 tokens x 4096 columns, top-8: 2.4 GB in 339 us,
-// 7.1 TB/s).  A decode batch has too few tokens
-// for that and sees the latency of a chain of loads instead: the list is fetched 128 entries at a time, eight rows are
-// on their way before the first is added, and blockIdx.y spreads a token's columns over several CTAs when there are few
-// tokens (3 tokens x 3072 columns, top-8: 10.4 -> 3.7 us; 128 tokens, 16 rows each: 17.4 -> 6.0 us).
+// Bound by the y_pos rows it reads (32768 tokens x 4096 columns, top-8: 2.4 GB in 366 us, the copy rate).  A decode batch
+// has too few tokens for that and sees the latency of a chain of loads instead: the list is fetched 128 entries at a time,
+// ROWS rows are on their way before the first is added, and blockIdx.y spreads a token's columns over several CTAs when
+// there are few tokens (cold caches; 3 tokens x 3072 columns, top-8: 10.4 -> 3.7 us; 128 tokens, 16 rows each:
+// 17.4 -> 6.0 us).
+template <int ROWS>
 __global__ void __launch_bounds__(128) combine_kernel(const __nv_bfloat16* __restrict__ y_pos,
                                                       const int32_t* __restrict__ table, int T, int n_cand, int H,
                                                       __nv_bfloat16* __restrict__ out) {
@@ -42,13 +43,13 @@ __global__ void __launch_bounds__(128) combine_kernel(const __nv_bfloat16* __res
   const int n = s_n;
   for (int h = (blockIdx.y * blockDim.x + threadIdx.x) * 8; h < H; h += gridDim.y * blockDim.x * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int r0 = 0; r0 < n; r0 += 8) {
-      uint4 raw[8];
+    for (int r0 = 0; r0 < n; r0 += ROWS) {
+      uint4 raw[ROWS];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < ROWS; ++j)
         if (r0 + j < n) raw[j] = __ldg(reinterpret_cast<const uint4*>(y_pos + static_cast<int64_t>(s_rows[r0 + j]) * H + h));
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < ROWS; ++j) {
         if (r0 + j >= n) break;
         const uint32_t w[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
 #pragma unroll
@@ -80,11 +81,16 @@ extern "C" int b200moe_combine(const void* y_pos_bf16, const int32_t* table, int
                   "combine: need T, n_cand > 0 and H %% 8 == 0");
   B200MOE_REQUIRE(n_cand <= kMaxCandidates, B200MOE_ERR_INVALID, "combine: at most %d candidates per row, got %d",
                   kMaxCandidates, n_cand);
-  // a CTA covers 1024 columns at a time: one per token once the tokens alone give every SM several
-  const int col_ctas = T >= 8 * sm_count() ? 1 : (H + 1023) / 1024;
-  B200MOE_CUDA_OK(launch_overlapped(combine_kernel, dim3(T, col_ctas), 128, static_cast<size_t>(n_cand) * sizeof(int32_t),
-                                    static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(y_pos_bf16), table,
-                                    T, n_cand, H, static_cast<__nv_bfloat16*>(out_bf16)));
+  // A CTA covers 1024 columns at a time: one per token once the tokens alone give every SM several.  Then occupancy hides
+  // the latency as well as loads in flight do, which cost registers (cold L2, 4096 tokens of two rows: 24.6 us with one
+  // row at a time, 26.0 with four, 30.7 with eight; 2531 tokens of four rows of 64: 25.6 with two, 21.5 with four, 22.5
+  // with eight; 32768 tokens of eight: 396, 366, 360).
+  const bool many = T >= 8 * sm_count();
+  const auto kernel = !many ? combine_kernel<8> : (n_cand <= 2 ? combine_kernel<1> : combine_kernel<4>);
+  B200MOE_CUDA_OK(launch_overlapped(kernel, dim3(T, many ? 1 : (H + 1023) / 1024), 128,
+                                    static_cast<size_t>(n_cand) * sizeof(int32_t), static_cast<cudaStream_t>(stream),
+                                    static_cast<const __nv_bfloat16*>(y_pos_bf16), table, T, n_cand, H,
+                                    static_cast<__nv_bfloat16*>(out_bf16)));
   B200MOE_LAUNCH_OK("combine_kernel");
   return B200MOE_OK;
 }
