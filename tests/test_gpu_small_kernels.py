@@ -103,7 +103,7 @@ def test_rmsnorm_odd_rows(T, H, offset, residual):
     assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-30).all())
 
 
-@pytest.mark.parametrize("T,n_cand,H", [(1, 1, 8), (3, 7, 1032), (2, 9, 3072), (5, 130, 2056), (1200, 17, 256)])
+@pytest.mark.parametrize("T,n_cand,H", [(1, 1, 8), (3, 7, 1032), (2, 9, 3072), (5, 130, 2056), (1200, 17, 256), (1300, 2, 1032)])
 def test_combine_lists(T, n_cand, H):
     L = _lib()
     rows = T * n_cand
