@@ -75,6 +75,8 @@ class MoELayer:
         st = _lib.stream_ptr()
         E, K, B, N, H, I = self.E, self.K, self.B, self.N, self.H, self.I
         w, ws = self.weights, self.ws
+        # timed one by one, a launch must not start in the one before
+        variant = self.gemm_variant | (_lib.GEMM_CHAINED if timers is None else 0)
 
         def timed(name, fn):
             if timers is None:
@@ -103,13 +105,13 @@ class MoELayer:
             "b200moe_grouped_gemm1_swiglu", _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(w.w1), _lib.ptr(w.w1_sf), w.w_format,
             _lib.ptr(w.bias_gu), _lib.ptr(self.b2e), _lib.ptr(self.cond), _lib.ptr(ws.tile_flags), N, B, E, H, I,
             self.act_fn.value, nan, nan, nan, nan, _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(ws.status) + 4,
-            self.gemm_variant | _lib.GEMM_CHAINED,
+            variant,
             None if self.clock_probe is None else _lib.ptr(self.clock_probe[0:]), st))
         timed("gemm2_scale", lambda: _lib.call(
             "b200moe_grouped_gemm2_scale", _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(w.w2), _lib.ptr(w.w2_sf), w.w_format,
             _lib.ptr(w.bias_d), _lib.ptr(self.b2e), _lib.ptr(self.cond), _lib.ptr(ws.tile_flags), _lib.ptr(self.tpi),
             T, N, B, E, H, I, _lib.ptr(self.aff), _lib.F32, 0, _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8,
-            self.gemm_variant | _lib.GEMM_CHAINED,
+            variant,
             None if self.clock_probe is None else _lib.ptr(self.clock_probe[2:]), st))
         timed("combine", lambda: _lib.call(
             "b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(self.inv), T, K, H, _lib.ptr(out), st))

@@ -85,6 +85,7 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
             ev.record()
             timers.setdefault(name, []).append(ev)
 
+    chained = _lib.GEMM_CHAINED if timers is None else 0  # timed one by one, a launch must not start in the one before
     mark("t0")
     # token-major quantise: ``table`` lists every token's positions, so a hidden row is read and quantised once
     # and stored to each of them (a position-major gather would read it once per expert the token goes to)
@@ -97,13 +98,13 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
               _lib.ptr(weights.w1_sf), weights.w_format, _lib.ptr(weights.bias_gu), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), n_blocks, block_size, E, H, I, act_fn, _clamp(gate_clamp[0]),
               _clamp(gate_clamp[1]), _clamp(up_clamp[0]), _clamp(up_clamp[1]), _lib.ptr(ws.mq), _lib.ptr(ws.m_sf),
-              _lib.ptr(ws.status) + 4, impl | (_lib.GEMM_CHAINED if flags_ready else 0), None, st)
+              _lib.ptr(ws.status) + 4, impl | (chained if flags_ready else 0), None, st)
     mark("t2")
     _lib.call("b200moe_grouped_gemm2_scale", _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(weights.w2),
               _lib.ptr(weights.w2_sf), weights.w_format, _lib.ptr(weights.bias_d), _lib.ptr(block_to_expert), _lib.ptr(conditions),
               _lib.ptr(ws.tile_flags), _lib.ptr(token_position_to_id), hidden_rows, n_blocks, block_size, E, H, I,
               _lib.ptr(affinities), _lib.F32 if affinities is None else _lib.dtype_code(affinities),
-              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8, impl | _lib.GEMM_CHAINED, None, st)
+              int(aff_per_row), _lib.ptr(ws.y_pos), _lib.ptr(ws.status) + 8, impl | chained, None, st)
     mark("t3")
     _lib.call("b200moe_combine", _lib.ptr(ws.y_pos), _lib.ptr(table), out.shape[0], table.shape[1], H, _lib.ptr(out), st)
     if check_status:
