@@ -780,7 +780,7 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             float v = __uint_as_float(raw[l][j]);
-            if constexpr (KIND == 1) v *= factor[0];
+            if constexpr (KIND == 1) v = __fmul_rn(v, factor[0]);  // rounded before the bias, never one fused step
             v += bias[0];
             if (clamp) v = fminf(fmaxf(v, c_lo), c_hi);
             column[j * kTurnPitch] = v;
@@ -855,7 +855,10 @@ grouped_mxfp8_gemm_kernel(const __grid_constant__ WeightMaps wmap, const __grid_
             for (int i = 0; i < 4; ++i) {
               float v0 = __uint_as_float(raw[l][(i >> 1) * 16 + g * 4 + (i & 1) * 2]);
               float v1 = __uint_as_float(raw[l][(i >> 1) * 16 + g * 4 + (i & 1) * 2 + 1]);
-              if constexpr (KIND == 1) { v0 *= factor[i]; v1 *= factor[i]; }
+              if constexpr (KIND == 1) {
+                v0 = __fmul_rn(v0, factor[i]);
+                v1 = __fmul_rn(v1, factor[i]);
+              }
               const __nv_bfloat162 b2 = __floats2bfloat162_rn((v0 + bias[i]) * a.x, (v1 + bias[i]) * a.y);
               m[i] = *reinterpret_cast<const uint32_t*>(&b2);
             }

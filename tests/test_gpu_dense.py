@@ -87,3 +87,38 @@ def test_dense_pre_scale_is_rejected_by_decode_and_mx_prefill():
         m.moe_tkg(torch.from_numpy(d["hidden"]).to(torch.bfloat16).cuda(), _w(d["gate_up"], "bf16"), _w(d["down"], "bf16"),
                   torch.from_numpy(d["aff"]).cuda(), torch.from_numpy(d["expert_index"]).cuda(), False,
                   expert_affinities_scaling_mode=m.ExpertAffinityScaleMode.PRE_SCALE)
+
+
+@pytest.mark.parametrize("variant", ["single", "pair"])
+@pytest.mark.parametrize("part", ["gate_up", "down"])
+def test_fp8row_factor_is_rounded_before_the_bias(part, variant):
+    """accumulator x factor is rounded to fp32, then the bias is added: with bias = -round(accumulator x factor) nothing
+    is left, exactly.  One fused step would leave the rounding error of the product.  The accumulators are small whole
+    numbers and every token is the same row, so both sides of the sum are known to the bit."""
+    import nki_library_b200 as m
+    from nki_library_b200 import _lib
+    from nki_library_b200.weights import prepare_dense
+    T, H, I, B = 40, 128, 64, 128
+    g = torch.Generator().manual_seed(5)
+    x = torch.randint(-3, 4, (1, H), generator=g).float()
+    w1 = torch.randint(-4, 5, (1, H, 2, I), generator=g).float()
+    w2 = torch.randint(-4, 5, (1, I, H), generator=g).float()
+    s1 = torch.rand((1, 2, I), generator=g) + 0.3
+    s2 = torch.rand((1, H), generator=g) + 0.3
+    acc1 = torch.einsum("h,hsi->si", x[0], w1[0])  # whole numbers far below 2^24
+    b_gu = -(acc1 * s1[0])[None]
+    b_d = torch.zeros((1, H))
+    if part == "down":
+        # silu(64) = 64 (exp(-64) vanishes beside 1) and up = 1: every intermediate is 64
+        s1[:], b_gu = 0.0, torch.stack([torch.full((I,), 64.0), torch.ones(I)])[None]
+        acc2 = 64.0 * w2[0].sum(0)
+        b_d = -(acc2 * s2[0])[None]
+    fp8 = [t.to(torch.float8_e4m3fn).cuda() for t in (w1, w2)]
+    w = prepare_dense(*fp8, *(t.contiguous().cuda() for t in (b_gu, b_d, s1, s2)))
+    tpi = torch.full((B,), -1, dtype=torch.int32, device="cuda")
+    tpi[:T] = torch.arange(T, device="cuda")
+    out = m.moe_cte(x.to(torch.bfloat16).cuda().expand(T, H).contiguous(), torch.ones((T, 1), device="cuda"), w, None, tpi,
+                    torch.zeros(1, dtype=torch.int32, device="cuda"), B, m.MoECTESpec(m.MoECTEImplementation.shard_on_i),
+                    skip_dma=m.SkipMode(True, False), _check_status=True,
+                    _impl=_lib.GEMM_NO_PAIR if variant == "single" else _lib.GEMM_FORCE_PAIR)
+    assert not out.any()
