@@ -371,9 +371,9 @@ RouterPlan plan_router(int T, int H, int E, int x_is_TH) {
   p.mw = 8 / p.nw;
   p.tm = 16 * p.mw;
   const int token_tiles = (T + p.tm - 1) / p.tm;
-  // At least two slabs per split: all of a split's loads are then in flight at once (the ring holds two or three), and
-  // the ranking still reads few partial sums.  Four slabs: 64-token decode 255.4 us, two: 253.5.
-  const int max_splits = (H + 2 * kKC - 1) / (2 * kKC);
+  // At least 256 hidden columns per split.  128 would shorten a decode batch's router by about 2 us (64 tokens, whole pass:
+  // 258.4 us with 256, 256.5 with 128), but add the products in another order, and with it change affinities and outputs.
+  const int max_splits = (H + 4 * kKC - 1) / (4 * kKC);
   int want = (2 * sm_count() + token_tiles - 1) / token_tiles;
   if (want < 1) want = 1;
   p.splits = want < max_splits ? want : max_splits;

@@ -241,3 +241,20 @@ def test_router_winner_lanes(act, mode, E, k):
     want = full if mode == "pre" else torch.zeros_like(full).scatter_(1, order, val)
     # a handful of fp32 operations per value, exponents of up to ~10: 1e-5 relative
     assert bool(((aff.double() - want).abs() <= 1e-5 * want + 1e-12).all())
+
+
+@pytest.mark.parametrize("T", [1, 16, 64])
+def test_router_sum_order(T):
+    """A split of the hidden axis holds at least 256 columns; inside one the products are added in fp32, the splits' sums in
+    order.  2^24 in the first split swallows a 1 that is added alone, not a 2: each later split holds two ones, 128 columns
+    apart."""
+    import nki_library_b200 as m
+    H, E = 1024, 8
+    x, w = torch.zeros((T, H), device="cuda"), torch.zeros((H, E), device="cuda")
+    x[:, 0], w[0] = 4096.0, 4096.0
+    for s in (256, 512, 768):
+        x[:, s], x[:, s + 128], w[s], w[s + 128] = 1.0, 1.0, 1.0, 1.0
+    logits, aff = torch.empty((T, E), device="cuda"), torch.empty((T, E), device="cuda")
+    idx = torch.empty((T, 2), dtype=torch.int32, device="cuda")
+    m.router_topk(x.to(torch.bfloat16), w.to(torch.bfloat16), None, logits, aff, idx, m.RouterActFnType.SOFTMAX, 2, 1, 0)
+    assert bool((logits == 2.0 ** 24 + 6).all())
