@@ -61,10 +61,11 @@ enum { B200MOE_W_E4M3 = 0, B200MOE_W_E5M2 = 1, B200MOE_W_E2M1 = 5 };
  *   B200MOE_GEMM_FORCE_PAIR  CTA pairs whatever the shape (default: when the block size is a multiple of 256, or
  *                            the block list holds two or more 128-position tiles per expert)
  *   B200MOE_GEMM_NO_SPLIT, B200MOE_GEMM_NO_OVERLAP  accepted and ignored: there is one launch per contraction
- *   B200MOE_GEMM_CHAINED     the launch may overlap the end of the kernel launched directly in front on this stream:
- *                            everything it reads but x (and, down, m) with their scales was complete before that kernel
- *                            was launched.  Only the quantisers, b200moe_all_expert_setup and the gate/up contractions
- *                            let a chained launch in early */
+ *   B200MOE_GEMM_CHAINED     the launch may overlap the end of the kernel launched directly in front on this stream.  Any
+ *                            kernel of this library may let it in early, so the launch directly in front may write
+ *                            nothing that this one reads but x (down: m) and its scales: block list, conditions, tile
+ *                            flags, token ids, affinities and weights come from earlier launches, and a status word
+ *                            that the launch in front uses is not this one's.  Ignored with clock_probe and SIMT */
 enum {
   B200MOE_IMPL_SIMT = 1,
   B200MOE_GEMM_TILE_N128 = 0x100,
@@ -241,7 +242,7 @@ int b200moe_prepare_gate_up_bias(const void* bias, int dtype, int layout, int E,
  * reference's block loop); tile_flags (NULL = all
  * tiles run; see b200moe_gather_quantize_mxfp8); token_position_to_id [n_blocks*B] and
  * hidden_rows (ids outside [0, hidden_rows) are pads, their rows are not written); status: device
- * int32[1], set non-zero if a kernel-internal wait ran out; impl: the per-call variant
+ * int32[1], cleared by the launch and set non-zero if a kernel-internal wait ran out; impl: the per-call variant
  * word, 0 = tcgen05 tensor-core kernel with tile shapes chosen by the library,
  * B200MOE_IMPL_SIMT = plain CUDA-core validation kernel (slow, same results up to
  * summation order), B200MOE_GEMM_* bits = restrictions on the tile shapes (below);

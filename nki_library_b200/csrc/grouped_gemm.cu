@@ -1217,8 +1217,9 @@ int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, 
                     (p.B % 256 == 0 || (impl & B200MOE_GEMM_FORCE_PAIR) || p.m_tiles_total >= 2 * p.E);
   p.max_n = pair ? 256 : 128;
   p.w_slab_bytes = nibbles ? kBlockK / 2 : kBlockK;
-  // (a gate/up launch that has to clear scale atoms first follows a memset, not a kernel)
-  p.chained = (impl & B200MOE_GEMM_CHAINED) != 0 && (epi == 1 || kind == 1 || p.I % 128 == 0);
+  // (a gate/up launch that has to clear scale atoms first follows a memset, not a kernel; a probed launch must not count
+  // the drain of the one in front)
+  p.chained = (impl & B200MOE_GEMM_CHAINED) != 0 && clock_probe == nullptr && (epi == 1 || kind == 1 || p.I % 128 == 0);
   WeightMaps wm;
   TokenMaps xm;
   CUtensorMap* const w_maps[4] = {&wm.rows128, &wm.rows64, &wm.rows32, &wm.rows16};

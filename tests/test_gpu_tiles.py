@@ -55,3 +55,35 @@ def test_tile_edges(variant, counts, B, H, I, holes):
     ref = run(_lib.IMPL_SIMT)
     got = run(_lib.GEMM_NO_PAIR if variant == "single" else _lib.GEMM_FORCE_PAIR)
     assert float((got - ref).abs().max() / ref.abs().max()) <= TOL
+
+
+def test_clock_probe_times_its_own_launch():
+    """A probed contraction does not start inside the launch in front, whose rest it would count.  In front stands a long
+    RMSNorm that leaves most SMs idle and lets chained launches in at once."""
+    from nki_library_b200 import _lib, pipeline
+    from nki_library_b200.layer import random_expert_weights
+    H, I = 128, 128
+    w = random_expert_weights(1, H, I, "cuda", seed=1)
+    ws = pipeline.BlockWorkspace(128, H, I, "cuda")
+    ws.xq.zero_()
+    ws.tile_flags.fill_(128)
+    b2e = torch.zeros(1, dtype=torch.int32, device="cuda")
+    probe = torch.zeros(2, dtype=torch.int64, device="cuda")
+    rows, cols = 32, 1 << 24
+    x = torch.zeros((rows, cols), dtype=torch.bfloat16, device="cuda")
+    out = torch.empty_like(x)
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    nan = float("nan")
+    for _ in range(2):
+        torch.cuda.synchronize()
+        ev[0].record()
+        _lib.call("b200moe_rmsnorm", _lib.ptr(x), None, None, _lib.F32, rows, cols, 0, 1e-6, _lib.ptr(out), None,
+                  _lib.stream_ptr())
+        _lib.call("b200moe_grouped_gemm1_swiglu", _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(w.w1), _lib.ptr(w.w1_sf),
+                  w.w_format, None, _lib.ptr(b2e), None, _lib.ptr(ws.tile_flags), 1, 128, 1, H, I, 0, nan, nan, nan, nan,
+                  _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(ws.status) + 4, _lib.GEMM_CHAINED, _lib.ptr(probe),
+                  _lib.stream_ptr())
+        ev[1].record()
+    torch.cuda.synchronize()
+    assert ws.status.tolist()[1] == 0
+    assert 0 < int(probe[1]) < 0.2e6 * ev[0].elapsed_time(ev[1])  # nanoseconds against a fifth of milliseconds
