@@ -115,8 +115,6 @@ __device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n
   if (tid == 0) { s.n_active = p.n_blocks; s.contiguous = 1; }
   for (int e = tid; e < p.E; e += nthr) { s.first_row[e] = 0; s.rows[e] = 0; s.start[e] = 0; }
   __syncthreads();
-  const int32_t* b2e = p.block_to_expert;
-  const int32_t* flags = p.tile_flags;
   const bool staged = p.n_blocks + p.m_tiles_total <= scratch_ints;
   for (int b = tid; b < p.n_blocks; b += nthr) {
     const int e = staged ? __ldcg(p.block_to_expert + b) : 0;
@@ -124,20 +122,18 @@ __device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n
     if (staged) scratch[b] = e;
     if (run == 0) atomicMin(&s.n_active, b);
   }
-  if (staged) {
-    if (p.tile_flags != nullptr) {
-      for (int t = tid; t < p.m_tiles_total; t += nthr) scratch[p.n_blocks + t] = __ldcg(p.tile_flags + t);
-      flags = scratch + p.n_blocks;
-    }
-    b2e = scratch;
-  }
+  const bool have_flags = p.tile_flags != nullptr;
+  if (staged && have_flags)
+    for (int t = tid; t < p.m_tiles_total; t += nthr) scratch[p.n_blocks + t] = __ldcg(p.tile_flags + t);
+  const auto b2e = [&](int b) { return staged ? scratch[b] : __ldcg(p.block_to_expert + b); };
+  const auto flags = [&](int t) { return staged ? scratch[p.n_blocks + t] : __ldcg(p.tile_flags + t); };
   __syncthreads();
   const int n_active = s.n_active;
   // start[] counts an expert's separate runs of blocks here, rows[] its 128-row tiles
   for (int b = tid; b < n_active; b += nthr) {
-    const int e = b2e[b];
+    const int e = b2e(b);
     if (e < 0 || e >= p.E) continue;
-    if (b == 0 || b2e[b - 1] != e) {
+    if (b == 0 || b2e(b - 1) != e) {
       s.first_row[e] = b * p.B;
       if (atomicAdd(&s.start[e], 1) > 0) s.contiguous = 0;
     }
@@ -147,17 +143,17 @@ __device__ __forceinline__ void build_sched(const GemmParams& p, Sched& s, int n
   const bool contiguous = s.contiguous;
   for (int e = tid; e < p.E && contiguous; e += nthr) {
     int live = s.rows[e], last = 128;
-    if (flags != nullptr && live > 0) {
+    if (have_flags && live > 0) {
       const int t0 = s.first_row[e] >> 7;
-      while (live > 0 && (last = flags[t0 + live - 1]) == 0) --live;
+      while (live > 0 && (last = flags(t0 + live - 1)) == 0) --live;
     }
     s.rows[e] = live > 0 ? (live - 1) * 128 + last : 0;
   }
   __syncthreads();
-  if (flags != nullptr && contiguous) {
+  if (have_flags && contiguous) {
     for (int t = tid; t < n_active * sub; t += nthr) {
-      if (flags[t] >= 128) continue;
-      const int e = b2e[t / sub];
+      if (flags(t) >= 128) continue;
+      const int e = b2e(t / sub);
       if (e < 0 || e >= p.E) continue;
       const int r = s.rows[e], end = s.first_row[e] + (r < 0 ? -r : r);
       if ((t + 1) * 128 < end && r > 0) atomicMin(&s.rows[e], -r);
