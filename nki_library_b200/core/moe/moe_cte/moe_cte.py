@@ -162,7 +162,7 @@ def moe_cte(
     table = torch.empty((rows, E), dtype=torch.int32, device=hidden.device)
     ws = pipeline.get_workspace(N * block_size, H, weights.I, hidden.device)
     _lib.call("b200moe_build_position_table_tiles", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
-              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
+              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), ws.stream)
     if rows != hidden_rows:
         table[hidden_rows:].fill_(-1)
     pipeline.run_blocks(hidden, hidden_rows, weights, tpi, b2e, conditions, block_size, aff, table, out,
@@ -208,7 +208,7 @@ def _moe_cte_dense(hidden_states, expert_affinities_masked, gate_up_proj_weight,
     table = torch.empty((rows, E), dtype=torch.int32, device=hidden.device)
     ws = pipeline.get_dense_workspace(N * block_size, H, weights.I, hidden.device)
     _lib.call("b200moe_build_position_table_tiles", _lib.ptr(tpi), _lib.ptr(b2e), _lib.ptr(conditions), N, block_size,
-              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
+              hidden_rows, E, _lib.ptr(table), _lib.ptr(ws.tile_flags), ws.stream)
     if rows != hidden_rows:
         table[hidden_rows:].fill_(-1)
     pipeline.run_blocks_dense(hidden, hidden_rows, weights, tpi, b2e, conditions, block_size, aff, table, out,

@@ -105,7 +105,7 @@ def moe_block_tkg(
         prequantized = (ws, layout)
         _lib.call("b200moe_rmsnorm_quantize_mxfp8", _lib.ptr(x), _lib.ptr(res), _lib.ptr(g), g_code, T, H, h_act,
                   float(eps), _lib.ptr(normed), _lib.ptr(residual_out), _lib.ptr(table), table.shape[1], n_pos,
-                  int(w.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(ws.tile_flags), _lib.stream_ptr())
+                  int(w.h_packed_order), _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(ws.tile_flags), ws.stream)
     else:
         _lib.call("b200moe_rmsnorm", _lib.ptr(x), _lib.ptr(res), _lib.ptr(g), g_code, T, H, h_act, float(eps),
                   _lib.ptr(normed), _lib.ptr(residual_out), _lib.stream_ptr())

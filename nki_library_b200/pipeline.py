@@ -9,6 +9,8 @@ the current CUDA stream; no host synchronisation happens unless
 from __future__ import annotations
 
 import math
+import threading
+from collections import OrderedDict
 from typing import Optional
 
 import torch
@@ -24,32 +26,56 @@ def _clamp(v):
 
 
 class BlockWorkspace:
-    """Device scratch for one (n_pos, H, I) shape, reused across calls."""
+    """Device scratch for one (n_pos, H, I) shape, reused across calls.  What a pass reads of it that pass has written,
+    rows without a token apart, so it need not start cleared (``zeroed``)."""
+    stream = None  # of a pool's workspace: the stream it belongs to
 
-    def __init__(self, n_pos: int, H: int, I: int, device):
+    def __init__(self, n_pos: int, H: int, I: int, device, zeroed: bool = True):
         lib = _lib.load_library()
+        new = torch.zeros if zeroed else torch.empty
         self.key = (n_pos, H, I, str(device))
         self.xq = torch.empty((n_pos, H), dtype=torch.uint8, device=device)
-        self.x_sf = torch.zeros(lib.b200moe_sf_bytes(n_pos, H), dtype=torch.uint8, device=device)
-        self.tile_flags = torch.zeros(math.ceil(n_pos / 128), dtype=torch.int32, device=device)
+        self.x_sf = new(lib.b200moe_sf_bytes(n_pos, H), dtype=torch.uint8, device=device)
+        self.tile_flags = new(math.ceil(n_pos / 128), dtype=torch.int32, device=device)
         self.mq = torch.empty((n_pos, I), dtype=torch.uint8, device=device)
-        self.m_sf = torch.zeros(lib.b200moe_sf_bytes(n_pos, I), dtype=torch.uint8, device=device)
+        self.m_sf = new(lib.b200moe_sf_bytes(n_pos, I), dtype=torch.uint8, device=device)
         self.y_pos = torch.empty((n_pos, H), dtype=torch.bfloat16, device=device)
         self.status = torch.zeros(4, dtype=torch.int32, device=device)
 
 
-_workspaces: dict = {}
+class _WorkspacePool(threading.local):
+    """Workspaces of the drop-in calls, kept between calls.  The launches of one call share theirs, so it belongs to one host
+    thread (two threads' launches may interleave on a stream) and one stream.  A thread keeps the five it used last and
+    gives them up when it ends; a workspace that is dropped returns to its stream's memory pool, behind the launches
+    that still use it.  While the stream is being captured a call gets one of its own: it comes from the graph's memory and
+    lives and is replayed with the graph, whatever eager calls do meanwhile."""
+    KEPT = 5
+
+    def __init__(self):
+        self.held = OrderedDict()
+
+    def get(self, make, n_pos: int, H: int, I: int, device):
+        stream = _lib.stream_ptr()
+        if torch.cuda.is_current_stream_capturing():
+            ws = make(n_pos, H, I, device, zeroed=False)
+            ws.stream = stream
+            return ws
+        key = (n_pos, H, I, device, stream)
+        ws = self.held.pop(key, None)
+        if ws is None:
+            if len(self.held) >= self.KEPT:
+                self.held.popitem(last=False)
+            ws = make(n_pos, H, I, device)
+            ws.stream = stream
+        self.held[key] = ws
+        return ws
+
+
+_workspaces = _WorkspacePool()
 
 
 def get_workspace(n_pos: int, H: int, I: int, device) -> BlockWorkspace:
-    key = (n_pos, H, I, str(device))
-    ws = _workspaces.get(key)
-    if ws is None:
-        if len(_workspaces) > 4:
-            _workspaces.clear()
-        ws = BlockWorkspace(n_pos, H, I, device)
-        _workspaces[key] = ws
-    return ws
+    return _workspaces.get(BlockWorkspace, n_pos, H, I, device)
 
 
 def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, token_position_to_id: torch.Tensor,
@@ -77,7 +103,7 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
     _lib.kernel_assert(hidden.dtype == torch.bfloat16 and hidden.shape[1] == H and hidden.is_contiguous(),
                        "hidden_states must be contiguous bf16 [rows, H]")
     ws = workspace or get_workspace(n_pos, H, I, hidden.device)
-    st = _lib.stream_ptr()
+    st = _lib.stream_ptr() if ws.stream is None else ws.stream
 
     def mark(name):
         if timers is not None:
@@ -115,26 +141,21 @@ def run_blocks(hidden: torch.Tensor, hidden_rows: int, weights: ExpertWeights, t
 
 class DenseWorkspace:
     """Device scratch of the dense (non-MX) path for one (n_pos, H, I) shape."""
+    stream = None
 
-    def __init__(self, n_pos: int, H: int, I: int, device):
+    def __init__(self, n_pos: int, H: int, I: int, device, zeroed: bool = True):
         self.x_pos = torch.empty((n_pos, H), dtype=torch.bfloat16, device=device)
         self.m = torch.empty((n_pos, I), dtype=torch.bfloat16, device=device)
         self.y_pos = torch.empty((n_pos, H), dtype=torch.bfloat16, device=device)
-        self.tile_flags = torch.zeros(math.ceil(n_pos / 128), dtype=torch.int32, device=device)
+        self.tile_flags = (torch.zeros if zeroed else torch.empty)(math.ceil(n_pos / 128), dtype=torch.int32, device=device)
         self.status = torch.zeros(4, dtype=torch.int32, device=device)
 
 
-_dense_workspaces: dict = {}
+_dense_workspaces = _WorkspacePool()
 
 
 def get_dense_workspace(n_pos: int, H: int, I: int, device) -> DenseWorkspace:
-    key = (n_pos, H, I, str(device))
-    ws = _dense_workspaces.get(key)
-    if ws is None:
-        if len(_dense_workspaces) > 4:
-            _dense_workspaces.clear()
-        ws = _dense_workspaces[key] = DenseWorkspace(n_pos, H, I, device)
-    return ws
+    return _dense_workspaces.get(DenseWorkspace, n_pos, H, I, device)
 
 
 def run_blocks_dense(hidden: torch.Tensor, hidden_rows: int, weights, token_position_to_id: torch.Tensor,
@@ -154,7 +175,7 @@ def run_blocks_dense(hidden: torch.Tensor, hidden_rows: int, weights, token_posi
     _lib.kernel_assert(hidden.dtype == torch.bfloat16 and hidden.shape[1] == H and hidden.is_contiguous(),
                        "hidden_states must be contiguous bf16 [rows, H]")
     ws = workspace or get_dense_workspace(n_pos, H, I, hidden.device)
-    st = _lib.stream_ptr()
+    st = _lib.stream_ptr() if ws.stream is None else ws.stream
     aff_code = _lib.F32 if affinities is None else _lib.dtype_code(affinities)
     _lib.call("b200moe_scatter_rows_bf16", _lib.ptr(hidden), min(hidden_rows, table.shape[0]), H, _lib.ptr(table),
               table.shape[1], n_pos, _lib.ptr(block_to_expert), block_size, E,
