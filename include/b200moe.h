@@ -185,7 +185,8 @@ int b200moe_build_position_table_tiles(const int32_t* token_position_to_id, cons
  * token_position_to_id [E_local * T_pad], block_to_expert [E_local * T_pad / B], pos_table [T, E_local].
  * local_affinities [T, E_local] fp32 (NULL = leave out): columns [E_local * r, E_local * (r + 1)) of the [T, E] table,
  * r = *rank_id (device integer of rank_bytes bytes; NULL = 0), multiplied by 0 where expert_index [T, K] (NULL = keep
- * all) does not name the expert; columns outside the table come back as NaN. */
+ * all; an entry of INT32_MIN is empty) does not name the expert.  Columns outside the table come back as NaN, and so do
+ * all columns of a token with an expert_index entry outside [0, E). */
 int b200moe_all_expert_setup(int T, int E_local, int B, int32_t* token_position_to_id, int32_t* block_to_expert,
                              int32_t* pos_table, const void* affinities, int aff_dtype, int E, const void* rank_id,
                              int rank_bytes, const int32_t* expert_index, int K, float* local_affinities,

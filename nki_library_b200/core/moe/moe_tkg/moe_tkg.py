@@ -60,6 +60,7 @@ def moe_tkg(
     the affinity columns sliced (and optionally masked by ``expert_index``) the
     way ``mask_expert_affinities`` does (core/moe/moe_tkg/moe_tkg_affinity_masking.py:31-117).
     ``is_all_expert_dynamic`` computes, per local expert, only the tokens whose masked affinity is non-zero.
+    A rank whose columns lie past the table and a token whose mask names an expert outside it give NaN rows.
     Weights are the reference's x4-packed MXFP8 tensors with their scales, or a
     prepared :class:`~nki_library_b200.weights.ExpertWeights` passed as
     ``expert_gate_up_weights``.  Non-MX weights -- 4-D ``[E_L, H, 2, I]`` bf16, or fp8 with the per-row factors
@@ -134,6 +135,7 @@ def moe_tkg(
         # local expert columns [E_L * rank_id, E_L * (rank_id + 1)), taken with a device-side index so that the
         # rank tensor never has to travel to the host (moe_tkg_affinity_masking.py:31-117)
         want_aff = post_scale or is_all_expert_dynamic
+        A(expert_affinities.device == dev, f"{_PREFIX} expert_affinities must be on the device of hidden_input")
         aff = local_affinities(expert_affinities, E_L, T, rank_id,
                                expert_index if mask_unselected_experts else None) if want_aff else None
         if is_all_expert_dynamic:
@@ -178,8 +180,14 @@ def all_expert_layout(T: int, E_L: int, device):
 
 def local_affinities(expert_affinities: torch.Tensor, E_L: int, T: int, rank_id, expert_index) -> torch.Tensor:
     """fp32 ``[T, E_L]``: this rank's columns of the affinity table, multiplied by 0 where ``expert_index`` (None = keep
-    all) does not name the expert.  The rank is read on the device and never travels to the host."""
+    all) does not name the expert.  The rank is read on the device and never travels to the host, so what cannot be checked
+    here shows in the result: columns past the table, and every column of a token with an expert id outside ``[0, E)``,
+    are NaN."""
     E = expert_affinities.shape[1]
+    dev = expert_affinities.device
+    _lib.kernel_assert((rank_id is None or rank_id.device == dev) and (expert_index is None or expert_index.device == dev),
+                       f"{_PREFIX} expert_affinities, expert_index and rank_id must be on one device")
+    _lib.kernel_assert(rank_id is None or rank_id.numel() > 0, f"{_PREFIX} rank_id must hold the rank")
     aff = expert_affinities.expand(T, E) if expert_affinities.shape[0] == 1 else expert_affinities
     _lib.kernel_assert(aff.shape[0] == T or (expert_index is None and aff.shape[0] > T),
                        f"{_PREFIX} expert_affinities must hold one row per token")
@@ -191,10 +199,12 @@ def local_affinities(expert_affinities: torch.Tensor, E_L: int, T: int, rank_id,
         rank = rank.to(torch.int64)
     idx, K = None, 0
     if expert_index is not None:
-        idx = expert_index if expert_index.dtype in (torch.int32, torch.uint32) else expert_index.to(torch.int32)
+        idx = expert_index
+        if idx.dtype not in (torch.int32, torch.uint32):
+            idx = (idx.clamp(-1, E) if idx.dtype == torch.int64 else idx).to(torch.int32)
         _lib.kernel_assert(idx.shape[0] <= T, f"{_PREFIX} expert_index must hold one row per token")
         if idx.shape[0] < T:  # a token without a row selects nothing
-            idx = torch.nn.functional.pad(idx.view(torch.int32), (0, 0, 0, T - idx.shape[0]), value=-1)
+            idx = torch.nn.functional.pad(idx.view(torch.int32), (0, 0, 0, T - idx.shape[0]), value=-2 ** 31)
         idx, K = idx.contiguous(), idx.shape[1]
     out = torch.empty((T, E_L), dtype=torch.float32, device=aff.device)
     _lib.call("b200moe_all_expert_setup", T, E_L, _BLOCK, None, None, None, _lib.ptr(aff), _lib.dtype_code(aff), E,

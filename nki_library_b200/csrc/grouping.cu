@@ -330,7 +330,8 @@ __global__ void position_table_kernel(const int32_t* tpi, const int32_t* block_t
 
 // All-expert decode: expert e of the rank's E_L holds tokens 0..T-1 in order, padded to whole blocks (tpi, b2e, table;
 // NULL = leave out), and sees the affinity columns [E_L * rank, E_L * (rank + 1)) of every token, zeroed where the
-// token did not select the expert (aff_out; NULL = leave out).  Columns past E read as NaN.  One launch in the place of
+// token did not select the expert (aff_out; NULL = leave out).  Columns past E read as NaN, as do all of a token that
+// selected an expert outside the table: neither can be refused without a host synchronisation.  One launch in the place of
 // some twenty element-wise ones: the decode block on 16 local experts, 128 tokens, spent 70 us
 // of device and 250 us of host time on those, 7 us on two of these.
 __global__ void all_expert_setup_kernel(int T, int E_L, int T_pad, int B, int32_t* tpi, int32_t* b2e, int32_t* table,
@@ -359,8 +360,11 @@ __global__ void all_expert_setup_kernel(int T, int E_L, int T_pad, int B, int32_
         v = load_as_float(aff, static_cast<int64_t>(t) * E + col, aff_dtype);
         if (selected != nullptr) {
           float keep = 0.0f;
-          for (int k = 0; k < K; ++k)
-            if (selected[static_cast<int64_t>(t) * K + k] == col) keep = 1.0f;
+          for (int k = 0; k < K; ++k) {
+            const int s = selected[static_cast<int64_t>(t) * K + k];
+            if (s == col) keep = 1.0f;
+            if ((s < 0 || s >= E) && s != INT32_MIN) v = __int_as_float(0x7fc00000);  // INT32_MIN: no entry
+          }
           v *= keep;
         }
       }

@@ -87,3 +87,16 @@ def test_cpu_tensors_are_rejected_not_silently_computed():
     with pytest.raises(AssertionError, match="pre-scale"):
         m.moe_tkg(torch.zeros(4, 512), None, None, torch.zeros(4, 8), torch.zeros(4, 2), False,
                   expert_affinities_scaling_mode=m.ExpertAffinityScaleMode.PRE_SCALE)
+
+
+def test_all_expert_affinities_refuse_mixed_devices_and_empty_ranks():
+    """Before anything is launched: a kernel would follow a pointer of another device."""
+    import importlib
+    mod = importlib.import_module("nki_library_b200.core.moe.moe_tkg.moe_tkg")
+    aff = torch.zeros(4, 8)
+    for rank, idx in ((torch.zeros(1, dtype=torch.int32, device="meta"), None),
+                      (None, torch.zeros((4, 2), dtype=torch.int32, device="meta"))):
+        with pytest.raises(AssertionError, match="one device"):
+            mod.local_affinities(aff, 4, 4, rank, idx)
+    with pytest.raises(AssertionError, match="rank_id must hold"):
+        mod.local_affinities(aff, 4, 4, torch.zeros((0, 1), dtype=torch.int32), None)

@@ -258,3 +258,22 @@ def test_router_sum_order(T):
     idx = torch.empty((T, 2), dtype=torch.int32, device="cuda")
     m.router_topk(x.to(torch.bfloat16), w.to(torch.bfloat16), None, logits, aff, idx, m.RouterActFnType.SOFTMAX, 2, 1, 0)
     assert bool((logits == 2.0 ** 24 + 6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64, torch.int16])
+def test_local_affinities_marks_what_it_cannot_refuse(dtype):
+    """Ids and ranks live on the device and are not read on the host: an expert outside the table makes its token's
+    affinities NaN, a rank outside it all of them; tokens without a row of ids select nothing."""
+    mod = importlib.import_module("nki_library_b200.core.moe.moe_tkg.moe_tkg")
+    T, E_L, E = 6, 4, 8
+    aff = torch.rand((T, E), device="cuda", generator=_gen(15))
+    idx = torch.tensor([[4, 5], [4, E], [-1, 6], [7, 30000], [0, 6]], device="cuda")
+    if dtype == torch.int64:
+        idx[3, 1] = 2 ** 32 + 5
+    rank = torch.tensor([[1]], dtype=torch.int32, device="cuda")
+    got = mod.local_affinities(aff, E_L, T, rank, idx.to(dtype))
+    assert bool(got[1:4].isnan().all())
+    want = torch.zeros((T, E_L), device="cuda")
+    want[0, :2], want[4, 2] = aff[0, 4:6], aff[4, 6]
+    assert torch.equal(got[[0, 4, 5]], want[[0, 4, 5]])
+    assert bool(mod.local_affinities(aff, E_L, T, rank + 1, None).isnan().all())
