@@ -42,7 +42,8 @@ def _run_gemm1(m, weights, x_np, b2e_np, B, impl, act=0, clamps=(None,) * 4):
     return ws.mq.cpu().numpy(), sf_atoms_to_rows(ws.m_sf.cpu().numpy(), n_pos, weights.I)
 
 
-@pytest.mark.parametrize("impl,tile_n", [(1, 256), (0, 256), (0, 128)])
+# CUDA cores, the library's choice, TILE_N128, NO_PAIR, FORCE_PAIR (one expert's two blocks are one tile of 256 tokens there)
+@pytest.mark.parametrize("impl,tile_n", [(1, 256), (0, 256), (0, 128), (0x200, 256), (0x400, 256)])
 def test_gate_up_swiglu_requantise_vs_oracle(impl, tile_n):
     import nki_library_b200 as m
     from nki_library_b200 import _lib
@@ -138,7 +139,7 @@ def test_moe_cte_cta_pair_mode(B, T, scatter):
     single = m.moe_cte(*args, _impl=_lib.GEMM_NO_PAIR, **kw)
     paired = m.moe_cte(*args, _impl=_lib.GEMM_FORCE_PAIR, **kw)
     paired2 = m.moe_cte(*args, _impl=_lib.GEMM_FORCE_PAIR, **kw)
-    # the same tiles with the left-over launch folded into half-empty pairs, and with it run strictly afterwards
+    # two bits of the variant word that are still accepted select nothing any more
     folded = m.moe_cte(*args, _impl=_lib.GEMM_FORCE_PAIR | _lib.GEMM_NO_SPLIT, **kw)
     serial = m.moe_cte(*args, _impl=_lib.GEMM_FORCE_PAIR | _lib.GEMM_NO_OVERLAP, **kw)
     assert torch.equal(paired, folded) and torch.equal(paired, serial)

@@ -57,6 +57,42 @@ def test_tile_edges(variant, counts, B, H, I, holes):
     assert float((got - ref).abs().max() / ref.abs().max()) <= TOL
 
 
+@pytest.mark.parametrize("variant", ["single", "pair"])
+@pytest.mark.parametrize("weights", ["e4m3", "e2m1", "bf16"])
+def test_many_tiles_per_cta(variant, weights):
+    """Every CTA walks several tiles of both contractions: token tiles wider than one accumulator between narrower ones, rows
+    of several experts through the same output buffers, a last round that single CTAs cut.  All outputs are compared."""
+    import nki_library_b200 as m
+    from nki_library_b200 import _lib
+    from nki_library_b200.layer import random_expert_weights
+    from nki_library_b200.weights import prepare_dense
+    counts, B, H, I = [256, 225, 224, 31, 480, 1, 449, 700, 0, 130, 65, 288] * 2, 256, 2048, 1024
+    tpi, b2e, T = _blocks(counts, B, False)
+    E = len(counts)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    if weights == "bf16":
+        w = prepare_dense(*((torch.randn(s, device="cuda", generator=g) * 0.02).to(torch.bfloat16)
+                            for s in ((E, H, 2, I), (E, I, H))))
+    else:
+        w = random_expert_weights(E, H, I, "cuda", seed=6, w_format=5 if weights == "e2m1" else 0)
+    w.bias_gu = torch.randn((E, 2 * I), device="cuda", generator=g) * 0.5
+    w.bias_d = torch.randn((E, H), device="cuda", generator=g) * 0.1
+    x = torch.randn((T, H), device="cuda", generator=g).to(torch.bfloat16)
+    aff = torch.rand((T, E), device="cuda", generator=g) + 0.5
+    spec = m.MoECTESpec(m.MoECTEImplementation.shard_on_block if weights == "bf16" else
+                        m.MoECTEImplementation.shard_on_block_mx)
+
+    def run(impl):
+        return m.moe_cte(x, aff.view(-1, 1), w, None, tpi, b2e, B, spec, skip_dma=m.SkipMode(True, False), _impl=impl,
+                         _check_status=True)
+
+    ref = run(_lib.IMPL_SIMT).float()
+    impl = _lib.GEMM_NO_PAIR if variant == "single" else _lib.GEMM_FORCE_PAIR
+    got = run(impl)
+    assert float((got.float() - ref).abs().max() / ref.abs().max()) <= TOL
+    assert torch.equal(run(impl), got)
+
+
 def test_clock_probe_times_its_own_launch():
     """A probed contraction does not start inside the launch in front, whose rest it would count.  In front stands a long
     RMSNorm that leaves most SMs idle and lets chained launches in at once."""
