@@ -5,9 +5,9 @@
 // expert's tokens are therefore cut into tiles of nearly equal width without padding them to 128, and one launch
 // covers every expert whatever its load.  With tokens as M (the earlier form of this kernel) an expert's last tile
 // cost a full 128 or 256 rows, odd tiles needed a second launch that streamed the weights again, and the output rows
-// left as 32-byte pieces.  Measured, whole layers, before -> now: 4096 tokens, 8 experts of 4096 x 14336, top-2: 1.36 ->
-// 1.23 ms; 8192 tokens, 256 experts of 7168 x 2048, top-8, skewed: 4.26 -> 3.91 ms; 2531 tokens, 64 experts of
-// 3072 x 1536, top-4 (160 tokens per expert): 0.53 -> 0.34 ms; 64 tokens on the first layer: 0.299 -> 0.291 ms.
+// left as 32-byte pieces.  Eager passes of the whole layer in a stream, earlier form -> this one: 4096 tokens, 8 experts of
+// 4096 x 14336, top-2: 1544 -> 1411 us; 8192 tokens, 256 experts of 7168 x 2048, top-8, skewed: 4568 -> 4410; 2531 tokens,
+// 64 experts of 3072 x 1536, top-4 (160 tokens per expert): 522 -> 351; 64 tokens on the first layer: 302 -> 287.
 //
 // What bounds it: with many tokens the L2 -> SM feed (a pair's tile of 256 x 256 needs 64 bytes per SM and tensor-pipe
 // clock; about 48 arrive) and the power cap; with few tokens the stream of weights from HBM.
@@ -1173,7 +1173,7 @@ int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, 
   B200MOE_REQUIRE(p.B > 0 && p.B % 128 == 0, B200MOE_ERR_INVALID, "block size must be a multiple of 128, got %d", p.B);
   B200MOE_REQUIRE(K % 32 == 0 && K >= 32, B200MOE_ERR_INVALID, "contraction length must be a multiple of 32, got %d", K);
   B200MOE_REQUIRE(kind == 0 || !(impl & B200MOE_GEMM_TILE_N128), B200MOE_ERR_INVALID,
-                  "the dense contraction has no 128-row weight tile");
+                  "TILE_N128 is an option of the MX contractions only; use NO_PAIR");
   B200MOE_REQUIRE(p.n_blocks > 0 && p.E > 0 && p.E <= kMaxExperts, B200MOE_ERR_INVALID,
                   "need at least one block and between 1 and %d experts", kMaxExperts);
   B200MOE_REQUIRE(p.status != nullptr, B200MOE_ERR_INVALID, "status pointer must not be null");
@@ -1204,11 +1204,16 @@ int run_gemm(int epi, const uint8_t* x, const uint8_t* w, GemmParams& p, int K, 
     B200MOE_LAUNCH_OK("simt_gemm_kernel");
     return B200MOE_OK;
   }
-  // CTA pairs (256 weight rows, up to 256 tokens per tile) once experts can hold more than one 128-row tile on average:
-  // each CTA then copies half of the token rows.  Below that a launch is bound by streaming the weights, and single CTAs
-  // (128 weight rows or fewer) spread the rows over the SMs in finer pieces.  Tiles of up to 256 tokens although only
-  // 224 leave room for a second accumulator: the 8192-token layer above took 4.2 ms with tiles of at most 224 and 3.9
-  // with 256, the 4096-token one 1.244 and 1.233 -- fewer operand bytes per MMA outweigh the drain at a tile's end.
+  // CTA pairs (256 weight rows, up to 256 tokens per tile; each CTA copies half of the token rows) when the block list has
+  // room for two 128-row tiles per expert, and for blocks of a multiple of 256 positions.  The host knows the list's
+  // length, not how many tokens an expert got, so the rule is a guess where the list is mostly padding: with few tokens per
+  // expert a launch is bound by streaming the weights, which single CTAs (128 weight rows or fewer) spread over the SMs in
+  // finer pieces.  Captured layers in us, blocks of 128 (which choose by length) / of 256 (always pairs): 8 experts of
+  // 4096 x 4096, top-2, 1 token per expert 66 / 104, 64 tokens 108 / 111, 128 tokens 136 / 125, 192 tokens 133 / 132;
+  // 64 experts of 3072 x 1536, top-4: 126 / 153, 211 / 216, 275 / 247, 282 / 295.
+  // Tiles of up to 256 tokens although only 224 leave room for a second accumulator: the 8192-token layer above took 7 %
+  // longer with tiles of at most 224, the 4096-token one 1 % -- fewer operand bytes per MMA outweigh the drain at a tile's
+  // end.
   const bool pair = !(impl & (B200MOE_GEMM_NO_PAIR | B200MOE_GEMM_TILE_N128)) && (sm_count() % 2 == 0) &&
                     (p.B % 256 == 0 || (impl & B200MOE_GEMM_FORCE_PAIR) || p.m_tiles_total >= 2 * p.E);
   p.max_n = pair ? 256 : 128;
