@@ -123,3 +123,47 @@ def test_clock_probe_times_its_own_launch():
     torch.cuda.synchronize()
     assert ws.status.tolist()[1] == 0
     assert 0 < int(probe[1]) < 0.2e6 * ev[0].elapsed_time(ev[1])  # nanoseconds against a fifth of milliseconds
+
+
+@pytest.mark.parametrize("variant", ["single", "pair"])
+@pytest.mark.parametrize("act", [0, 3])
+def test_gate_up_of_extreme_products(variant, act):
+    """MX blocks of gate/up products that are zero, subnormal, huge, infinite or NaN.  The weights are zero, so the biases
+    are the gates and ups; scales and codes against the CUDA-core kernel (values are no rounding ties of either)."""
+    from nki_library_b200 import _lib, pipeline
+    from nki_library_b200.weights import ExpertWeights
+    E, H, I, B = 7, 128, 128, 256
+    f = dict(dtype=torch.float32, device="cuda")
+    j = torch.arange(I, **f)
+    gate, up = (j % 13 - 6.1).repeat(E, 1), (j % 7 - 2.9).repeat(E, 1)
+    gate[1, 37] = float("nan")
+    up[2, 5] = float("inf")
+    gate[2, 70] = float("-inf")
+    gate[3] = 0.0
+    gate[4] = 3e-39
+    gate[5], up[5] = 1.5e30, 2.5e8
+    up[6, 64:96] = 1e-38
+    bias = torch.stack([gate, up], 1).view(E, 2, I // 32, 32).transpose(1, 2).reshape(E, 2 * I).contiguous()
+    lib = _lib.load_library()
+    zeros = [torch.zeros(n, dtype=torch.uint8, device="cuda") for n in
+             (E * 2 * I * H, E * lib.b200moe_sf_bytes(2 * I, H), E * H * I, E * lib.b200moe_sf_bytes(H, I))]
+    w = ExpertWeights(E, H, I, *zeros, bias, None, False)
+    b2e = torch.arange(E, dtype=torch.int32, device="cuda")
+    nan = float("nan")
+
+    def run(impl):
+        ws = pipeline.BlockWorkspace(E * B, H, I, "cuda")
+        for t in (ws.xq, ws.mq):
+            t.zero_()
+        ws.tile_flags.fill_(128)
+        _lib.call("b200moe_grouped_gemm1_swiglu", _lib.ptr(ws.xq), _lib.ptr(ws.x_sf), _lib.ptr(w.w1), _lib.ptr(w.w1_sf),
+                  w.w_format, _lib.ptr(w.bias_gu), _lib.ptr(b2e), None, _lib.ptr(ws.tile_flags), E, B, E, H, I, act, nan, nan,
+                  nan, nan, _lib.ptr(ws.mq), _lib.ptr(ws.m_sf), _lib.ptr(ws.status) + 4, impl, None, _lib.stream_ptr())
+        assert ws.status.tolist()[1] == 0
+        code = ws.mq & 0x7F
+        return torch.where(code == 0x7F, code, ws.mq), ws.m_sf  # a NaN's sign says nothing
+
+    ref = run(_lib.IMPL_SIMT)
+    got = run(_lib.GEMM_NO_PAIR if variant == "single" else _lib.GEMM_FORCE_PAIR)
+    assert torch.equal(got[1], ref[1])
+    assert torch.equal(got[0], ref[0])
