@@ -56,9 +56,9 @@ WORKLOADS = {
 # DRAM bytes (read + write) per launch of the dominant kernel, from the ncu captures summarised under
 # profiles/ (file named beside each figure; null where no capture of the current kernel exists).
 NCU_TRAFFIC = {
-    "mixtral_prefill": {"bytes": 1.136e9, "from": "profiles/grouped_mxfp8_gemm_mixtral_prefill.md (gate/up launch, captured "
+    "mixtral_prefill": {"bytes": 1.128e9, "from": "profiles/grouped_mxfp8_gemm_mixtral_prefill.md (gate/up launch, captured "
                         "on this workload at full size)"},
-    "mixtral_decode": {"bytes": 978.9e6, "from": "profiles/grouped_mxfp8_gemm_mixtral_decode.md (gate/up launch, captured "
+    "mixtral_decode": {"bytes": 978.6e6, "from": "profiles/grouped_mxfp8_gemm_mixtral_decode.md (gate/up launch, captured "
                        "on this workload at full size)"},
 }
 
